@@ -86,14 +86,9 @@ RC_HD uint64_t rc_f64_as_u64(double d) {
 typedef struct rc_u32x4 { uint32_t x, y, z, w; } rc_u32x4;
 
 RC_HD void rc_mulhilo32(uint32_t a, uint32_t b, uint32_t *hi, uint32_t *lo) {
-#if defined(__CUDA_ARCH__)
-    *hi = __umulhi(a, b);
-    *lo = a * b;
-#else
     uint64_t p = (uint64_t)a * (uint64_t)b;
     *hi = (uint32_t)(p >> 32);
     *lo = (uint32_t)p;
-#endif
 }
 
 /* One Philox4x32 bijection with 10 rounds; key schedule bumps (W0, W1)
@@ -178,11 +173,20 @@ RC_HD float rc_expf(float x) {
  * Arguments are clamped to [-87, 88] (e^-87 - 1 rounds to -1). */
 RC_HD float rc_expm1f(float x) {
     x = fminf(fmaxf(x, -87.0f), 88.0f);
+#if defined(__CUDA_ARCH__)
+    /* rintf and 2^n without conversion instructions: for |y| < 2^22 adding
+     * 1.5 2^23 rounds y to the nearest integer (ties to even, as rintf), which
+     * then stands in the low mantissa bits */
+    float t = x * RC_LOG2E_F + 12582912.0f;
+    float n = t - 12582912.0f;
+    float s = rc_u32_as_f32((rc_f32_as_u32(t) << 23) + 0x3f800000u);
+#else
     float n = rintf(x * RC_LOG2E_F);
+    float s = rc_exp2i_f((int)n);
+#endif
     /* n * ln2_hi is exact, so the inner fma is the exact x - n ln2_hi */
     float r = fmaf(-n, RC_LN2_LO_F, fmaf(-n, RC_LN2_HI_F, x));
     float p = rc_expm1_poly_f(r);
-    float s = rc_exp2i_f((int)n);
     return fmaf(s, p, s - 1.0f);
 }
 

@@ -37,9 +37,11 @@
 namespace rc {
 
 constexpr int kWarp = 32;
-constexpr int kRing = 64;    // per-warp ring of emitted bundles (two waves)
+constexpr int kRefill = 11;  // emitted bundles waiting below which a warp emits the next wave
+constexpr int kRing = kRefill - 1 + kWarp;  // per-warp ring of emitted bundles: those, and a wave
+constexpr int kTileBufs = 3;  // tiles a warp has in flight (tile_bufs)
 constexpr int kGuide = 256;  // buckets of the band-CDF guide tables
-constexpr int kFeedIdle = 14; // idle lanes that make a warp leave its step loop to take new bundles
+constexpr int kFeedIdle = 16; // idle lanes that make a warp leave its step loop to take new bundles
 constexpr int kTurnGather = 5; // lanes waiting at scattering events that make a warp draw their turns
 constexpr int kChunkMax = 8;  // tiles a warp claims per work-queue fetch (guided: fewer near the end)
 constexpr int kPhaseGuide = 64;  // phase-CDF guide buckets per band (scattering turns)
@@ -53,7 +55,7 @@ struct DLevel {
     int rx, ry, rz;           // ratio to the next (coarser) level
     unsigned mrx, mry, mrz;   // floor(2^32 / r) + 1 (0 for r = 1): (n + r - 1) / r as a multiply-high
     const R *xu, *yu, *zu;    // faces (views into DSolve::faces)
-    const uint16_t *P;        // table coordinate of every cell, i fastest (see cell_index);
+    const uint16_t *P;        // table coordinate of every cell and its halo (see cell_index);
                               // a view into DSolve::Pall
     const uint16_t *Pw[6];    // wall emission temperature coordinates (or null)
 };
@@ -81,9 +83,9 @@ struct DScalars {
 
 template <typename R>
 struct DSolve {
-    // what a step reads of its level, two 16-byte loads:
-    // lva = offsets of xu, yu, zu in faces and of the coordinates in Pall;
-    // lvb = (im, jm, km, maxs)
+    // what entering a level needs of it, two 16-byte loads:
+    // lva = (offset of xu in faces, offset of the coordinates in Pall, im, jm);
+    // lvb = (km, maxs, bits of dy, bits of dz): face j of y lies at j dy
     int4 lva[RC_MAX_LEVELS], lvb[RC_MAX_LEVELS];
     const R *faces;           // every level's xu | yu | zu, one after the other
     const uint16_t *Pall;     // every level's table coordinates, one after the other
@@ -128,6 +130,10 @@ struct DSolve {
     // multiply-high reciprocals of the item decomposition divisors
     unsigned long long mg_nchunk, mg_nvar, mg_imax, mg_jmax, mg_nwc;
     unsigned long long nwc;   // jmax * kloc
+    // 32-bit reciprocals of nVar, imax, jmax (tile_item); small_div: all three are at most 2^15
+    unsigned m_nvar, m_imax, m_jmax;
+    int small_div;
+    long long steps_to[RC_MAX_LEVELS];  // step budgets of the levels up to and including each
     uint32_t key0, key1;
     long long tile_base;      // first tile of this launch within the solve (server quanta)
     // extents for the bounds-checked build
@@ -140,9 +146,6 @@ struct DSolve {
 // extent: an index outside [0, n) sets status bit 3 and the first offending
 // site in DScalars::bad_site, and is replaced by 0 so the access stays
 // inside the array.  Nothing traps.
-#ifndef RC_CHECKED
-#define RC_CHECKED 0
-#endif
 enum RcSite : int {
     SITE_FACE = 1, SITE_PYRAMID, SITE_ROW, SITE_IBW, SITE_WALL_T, SITE_WALL_ROW, SITE_CENTRE, SITE_EMIT_T,
     SITE_WALL_EMIT_T, SITE_FACE_SHIFT, SITE_EMIT_ROW, SITE_DEN, SITE_IBM, SITE_PROBG, SITE_PARTIAL, SITE_LEVEL,
@@ -156,8 +159,10 @@ __device__ __forceinline__ long long rc_ix(long long i, long long n, int site, D
     return 0;
 }
 #define RC_IX(i, n, site, S) rc_ix((long long)(i), (long long)(n), (site), (S).sc)
+#define RC_IX_IF(go, i, n, site, S) ((go) ? RC_IX(i, n, site, S) : 0)
 #else
 #define RC_IX(i, n, site, S) (i)
+#define RC_IX_IF(go, i, n, site, S) (i)  // the lanes without `go` do not use the address
 #endif
 
 // ---------------------------------------------------------------------------
@@ -217,17 +222,40 @@ __device__ __forceinline__ KIRow<double> load_row(const KIRow<double> *p) {
     return r;
 }
 
-// Fraction of a table coordinate: (q mod 256) / 256, exact.
-template <typename R>
-__device__ __forceinline__ R coord_frac(int q) {
-    return (R)(q & 255) * (R)0.00390625;
+// The same by the lanes with `go` only; the others get anything.
+__device__ __forceinline__ void load_row_if(bool go, const KIRow<float> *p, KIRow<float> &r) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        : "=f"(r.k0), "=f"(r.ib0), "=f"(r.k1), "=f"(r.ib1)
+        : "l"(p), "r"((int)go));
+}
+__device__ __forceinline__ void load_row_if(bool go, const KIRow<double> *p, KIRow<double> &r) {
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.global.nc.v2.f64 {%0, %1}, [%4];\n\t"
+        "@p ld.global.nc.v2.f64 {%2, %3}, [%4+16];\n\t}"
+        : "=&d"(r.k0), "=&d"(r.ib0), "=&d"(r.k1), "=&d"(r.ib1)
+        : "l"(p), "r"((int)go));
 }
 
-// Offset of cell (i,j,k) (1-based) in an im x jm x km array, i fastest.
+// A level's words of the descriptor: from the kernel's parameters (constant
+// memory) when the launch marches one solve, else from device memory.
+template <bool ONE>
+__device__ __forceinline__ int4 load_desc(const int4 *p) {
+    if constexpr (ONE) return *p;
+    else return __ldg(p);
+}
+
+// Fraction of a table coordinate: (q mod 256) / 256, exact: the low byte in
+// the mantissa of 2^15 (unit 2^-8), 2^15 subtracted.
+template <typename R>
+__device__ __forceinline__ R coord_frac(int q) {
+    return (R)(__int_as_float(__byte_perm(q, 0x47000000, 0x7440)) - 32768.0f);
+}
+
+// Offset of cell (i,j,k) (1-based) of a level of im x jm cells per plane, i
+// fastest, one halo cell on every side (halo_code).
 // (A 4x4x4-brick layout was measured 2-3% slower: its index arithmetic
 // costs more issue slots than its locality saves in L1 misses.)
-__device__ __forceinline__ int cell_index(int i, int j, int k, int im, int jm) {
-    return (i - 1) + im * ((j - 1) + jm * (k - 1));
+__host__ __device__ __forceinline__ int cell_index(int i, int j, int k, int im, int jm) {
+    return i + (im + 2) * (j + (jm + 2) * k);
 }
 
 // Linear interpolation in temperature along one table column at a clamped
@@ -273,24 +301,32 @@ __device__ __forceinline__ int guided_index(const R *cdf, const int *guide, int 
     return u == (R)1 ? n - 1 : b;
 }
 
+// Index of a uniform u on a short non-decreasing cumulative table: the number
+// of its entries (the last left out) at or below u, the index the bisection
+// returns, from independent loads.
+template <typename R>
+__device__ __forceinline__ int count_index(const R *cdf, int n, R u) {
+    int g = 0;
+#pragma unroll 4
+    for (int d = 0; d < n - 1; ++d) g += !(u < cdf[d]);
+    return u == (R)1 ? n - 1 : g;
+}
+constexpr int kCountMax = 16;  // g points up to which counting replaces the bisection
+
 // Band and g point of an emitted bundle from its two uniforms: fluid bundles
 // (kind 0) search the band CDF at the table row nearest Tmax and then the
 // g CDF of that band and row (find_band, mc_gpu_noint.cu:1103-1169); wall
 // bundles (kind 1, 2) the Planck-only wall band CDF and the constant g CDF
-// probq (find_bandS :1170-1233, with the wall CDF's own edge rule).
+// probq (find_bandS :1170-1233, with the wall CDF's own edge rule).  The
+// fluid's tables are checked to be non-decreasing when they are set; probq
+// is not, so it keeps the bisection.
 template <typename R>
-__device__ __forceinline__ void select_band_g(const DSolve<R> &S, int kind, R u_b, R u_g, int &nb, int &g) {
-    if (kind == 0) {
-        nb = (int)RC_IX(guided_index(S.cdf_f, S.guide_f, S.nB, u_b), S.nB, SITE_CDF, S);
-        g = (S.nQ > 1)
-                ? bisect(S.probg + RC_IX(((size_t)S.row * S.nB + nb) * S.nQ, (long long)S.nT * S.nB * S.nQ,
-                                         SITE_PROBG, S),
-                         S.nQ, u_g)
-                : 0;
-    } else {
-        nb = (int)RC_IX(guided_index(S.cdf_s, S.guide_s, S.nB, u_b), S.nB, SITE_CDF, S);
-        g = (S.nQ > 1) ? bisect(S.probq, S.nQ, u_g) : 0;
-    }
+__device__ __forceinline__ void select_band_g(const DSolve<R> &S, int row, int kind, R u_b, R u_g, int &nb, int &g) {
+    const bool wall = kind != 0;
+    nb = (int)RC_IX(guided_index(wall ? S.cdf_s : S.cdf_f, wall ? S.guide_s : S.guide_f, S.nB, u_b), S.nB, SITE_CDF, S);
+    const R *cg = S.probg + RC_IX(((size_t)row * S.nB + nb) * S.nQ, (long long)S.nT * S.nB * S.nQ, SITE_PROBG, S);
+    g = S.nQ == 1 ? 0 : S.nQ <= kCountMax ? count_index(cg, S.nQ, u_g) : bisect(cg, S.nQ, u_g);
+    if (wall) g = S.nQ > 1 ? bisect(S.probq, S.nQ, u_g) : 0;
 }
 
 // A bundle after emission, placed at its start point: position, cell,
@@ -303,6 +339,14 @@ struct alignas(16) Emitted {
     int nbg;   // nb | g << 20
 };
 
+// A traced ray.  What a step reads is kept ready in registers: the exit face
+// of every axis (x: its coordinate fx and its index fi in DSolve::faces; y, z:
+// the index as a float and the level's spacing, whose product is the face
+// coordinate exactly as the grid builds it), the cell's offset in
+// DSolve::Pall with the signed offsets of the three possible neighbours, and
+// the cell's table coordinate.  A step moves one of the three axes, so it
+// loads one coordinate (and one x face) for the step after it, early enough
+// that the absorption of the current step hides their latency.
 template <typename R>
 struct Ray {
     R xp, yp, zp;
@@ -310,12 +354,26 @@ struct Ray {
     R isx, isy, isz;
     R tra;
     R Ibmax, ratioI, invTi4, tol;
-    const KIRow<R> *kicol;
-    int ic, jc, kc;
-    int lev, counter;
-    int nb;
+    R dI;                 // Ib / Ib(Ti) - 1 of the last step (the cutoff deposit of retire_ray)
+    R fx;
+    int fi;
+    float fj, fk, dy, dz;
+    int cidx, dx, dj, dk; // cell offset in Pall, offsets of the neighbours through the exit faces
+    int q;                // coordinate of the cell, the halo code beyond a wall
+    int kio;              // first table row of the bundle's band and g point
+    int ln;               // band | level << 20
+    int rem;              // steps left on the level
     double De;
 };
+// Coordinates of the halo cells around every level say what the wall between
+// does with a ray (256 table rows end at 65280): reflect it, let it re-enter
+// through the opposite face, or end it (kBlack + wall: black walls, and any
+// other type, whose rays are lost).
+constexpr int kSpecular = 0xfff0, kPeriodic = 0xfff1, kBlack = 0xfff8;
+
+__host__ __device__ __forceinline__ int halo_code(int wtype, int w) {
+    return wtype == 1 ? kPeriodic : wtype == 3 ? kSpecular : kBlack + w;
+}
 
 // Philox counter of one bundle: (h, v | kind << 24, cell, 0).
 __device__ __forceinline__ rc_u32x4 bundle_draws(uint32_t key0, uint32_t key1, int h, int v, int kind, uint32_t cell) {
@@ -335,80 +393,81 @@ __device__ __forceinline__ rc_u32x4 bundle_draws(uint32_t key0, uint32_t key1, i
 // OERM weights: invTi4 = 1/I_b(Ti); ratioI = (I_b(Ti) k(Ti)) / (I_b(Tmax)
 // k(Tmax)) for the fluid (the reference's ((1/invTi4)/Ib(Tmax))*k(Ti)/
 // k(Tmax), :180-186) and I_b(Ti)/I_b(Tmax) for walls (:1421-1424).
+// S: the solve's descriptor; row: its run-time table row nearest Tmax.
 template <typename R>
-__device__ __forceinline__ bool emit_bundle(Emitted<R> &e, const DSolve<R> &S, int kind, int i, int j, int k, int v,
-                                            int h) {
-    const uint32_t cell = (kind == 0)
-                              ? (uint32_t)((i - 1) + S.imax * ((j - 1) + S.jmax * (k - 1)))
-                              : (uint32_t)((j - 1) + S.jmax * (k - 1));
-    rc_u32x4 d = bundle_draws(S.key0, S.key1, h, v, kind, cell);
+__device__ __forceinline__ bool emit_bundle(Emitted<R> &e, const DSolve<R> &S, int row, int kind, int i, int j, int k,
+                                            int v, int h) {
+    // one path for cells and walls (values selected): a warp's wave runs it
+    // together, whatever its bundles are
+    const bool wall = kind != 0, east = kind == 2;
+    const uint32_t jk = (uint32_t)((j - 1) + S.jmax * (k - 1));
+    const uint32_t cell = wall ? jk : (uint32_t)(i - 1) + (uint32_t)S.imax * jk;
+    const rc_u32x4 d = bundle_draws(S.key0, S.key1, h, v, kind, cell);
     const R u_phi = (R)rc_u01(d.x), u_mu = (R)rc_u01(d.y), u_b = (R)rc_u01(d.z), u_g = (R)rc_u01(d.w);
     R sp, cp;
     RT<R>::sincos2pi_(u_phi, &sp, &cp);
-    int Pi;
-    int nb, g, ic = i;
-    R st;
-    if (kind == 0) {
-        // isotropic: cos(theta) = 1 - 2u (emiss_ang, :1077-1084)
-        const R mu = (R)1 - (R)2 * u_mu;
-        st = RT<R>::sqrt_(((R)1 - mu) * ((R)1 + mu));
-        e.sx = mu;
-        select_band_g(S, 0, u_b, u_g, nb, g);
-        const DLevel<R> &L0 = S.lev[0];
-        Pi = L0.P[RC_IX(cell_index(i, j, k, L0.im, L0.jm), (long long)L0.im * L0.jm * L0.km, SITE_EMIT_T, S)];
-    } else {
-        // Lambertian: theta = acos(1 - 2u)/2 (+pi/2 on the east wall)
-        // (emiss_angS, :1093-1102), i.e. cos = sqrt(1-u) / -sqrt(u).
-        const int bound = kind - 1;
-        if (bound == 0) {
-            e.sx = RT<R>::sqrt_((R)1 - u_mu);
-            st = RT<R>::sqrt_(u_mu);
-        } else {
-            e.sx = -RT<R>::sqrt_(u_mu);
-            st = RT<R>::sqrt_((R)1 - u_mu);
-        }
-        select_band_g(S, kind, u_b, u_g, nb, g);
-        Pi = S.Pw0[bound][RC_IX((k - 1) * S.jmax + (j - 1), (long long)S.kmax * S.jmax, SITE_WALL_EMIT_T, S)];
-        ic = (bound == 0) ? 1 : S.imax;
-    }
+    // cell, isotropic: cos(theta) = 1 - 2u (emiss_ang, :1077-1084); wall,
+    // Lambertian: theta = acos(1 - 2u)/2 (+pi/2 on the east wall)
+    // (emiss_angS, :1093-1102), i.e. cos = sqrt(1-u) / -sqrt(u)
+    const R mu = (R)1 - (R)2 * u_mu, um1 = (R)1 - u_mu;
+    const R st = RT<R>::sqrt_(wall ? (east ? um1 : u_mu) : ((R)1 - mu) * ((R)1 + mu));
+    e.sx = mu;
+    if (wall) e.sx = east ? -RT<R>::sqrt_(u_mu) : RT<R>::sqrt_(um1);
     e.sy = st * cp;
     e.sz = st * sp;
-    if (kind == 0) {
-        if (e.sx == (R)0) e.sx = (R)1e-10;  // :132-137
-        if (e.sy == (R)0) e.sy = (R)1e-10;
-        if (e.sz == (R)0) e.sz = (R)1e-10;
-    } else {
-        const int bound = kind - 1;
-        if (RT<R>::fabs_(e.sx) <= (R)1e-10) e.sx = (R)(1 - 2 * bound) * (R)1e-10;  // :1395-1400
-        if (RT<R>::fabs_(e.sy) <= (R)1e-10) e.sy = (R)((e.sy > (R)0) - (e.sy <= (R)0)) * (R)1e-10;
-        if (RT<R>::fabs_(e.sz) <= (R)1e-10) e.sz = (R)((e.sz > (R)0) - (e.sz <= (R)0)) * (R)1e-10;
-    }
+    // components floored (:132-137, walls :1395-1400)
+    const R tiny = wall ? (R)1e-10 : (R)0;
+    if (RT<R>::fabs_(e.sx) <= tiny) e.sx = (R)(east ? -1 : 1) * (R)1e-10;
+    if (RT<R>::fabs_(e.sy) <= tiny) e.sy = (R)(wall && !(e.sy > (R)0) ? -1 : 1) * (R)1e-10;
+    if (RT<R>::fabs_(e.sz) <= tiny) e.sz = (R)(wall && !(e.sz > (R)0) ? -1 : 1) * (R)1e-10;
+    int nb, g;
+    select_band_g(S, row, kind, u_b, u_g, nb, g);
+    const int Pi = wall ? S.Pw0[east][RC_IX(jk, (long long)S.kmax * S.jmax, SITE_WALL_EMIT_T, S)]
+                        : S.Pall[RC_IX(S.lva[0].y + cell_index(i, j, k, S.imax, S.jmax), S.n_P, SITE_EMIT_T, S)];
+    const int ic = wall ? (east ? S.imax : 1) : i;
     e.nbg = nb | (g << 20);
     e.ij = ic | (j << 16);
     e.kk = k | (kind << 16);
     // OERM weights
-    const KIRow<R> row =
-        S.ki[RC_IX(((size_t)nb * S.nQ + g) * S.nT + (Pi >> 8), (long long)S.nB * S.nQ * S.nT, SITE_EMIT_ROW, S)];
+    const KIRow<R> ki =
+        load_row(S.ki + RC_IX(((size_t)nb * S.nQ + g) * S.nT + (Pi >> 8), (long long)S.nB * S.nQ * S.nT, SITE_EMIT_ROW, S));
     const R fr = coord_frac<R>(Pi);
-    const R Ib_i = RT<R>::lerp_(row.ib0, row.ib1, fr);
-    if (!(Ib_i > (R)0)) return false;
+    const R Ib_i = RT<R>::lerp_(ki.ib0, ki.ib1, fr);
+    const R k_i = RT<R>::lerp_(ki.k0, ki.k1, fr);
+    const R den = wall ? S.ibm[RC_IX(nb, S.nB, SITE_IBM, S)]
+                       : S.den_f[RC_IX((size_t)nb * S.nQ + g, (long long)S.nB * S.nQ, SITE_DEN, S)];
     e.invTi4 = (R)1 / Ib_i;
-    if (kind == 0) {
-        const R k_i = RT<R>::lerp_(row.k0, row.k1, fr);
-        const R den = S.den_f[RC_IX((size_t)nb * S.nQ + g, (long long)S.nB * S.nQ, SITE_DEN, S)];
-        if (!(den > (R)0)) return false;
-        e.ratioI = (Ib_i * k_i) / den;
-    } else {
-        const R den = S.ibm[RC_IX(nb, S.nB, SITE_IBM, S)];
-        if (!(den > (R)0)) return false;
-        e.ratioI = Ib_i / den;
-    }
-    return true;
+    e.ratioI = (wall ? Ib_i : Ib_i * k_i) / den;
+    return Ib_i > (R)0 && den > (R)0;
 }
 
-// Ray state of an emitted bundle.
+// What a step of a ray in cell c of the level (A, B) reads: see Ray.
 template <typename R>
-__device__ __forceinline__ void place_bundle(Ray<R> &r, const DSolve<R> &S, const Emitted<R> &e) {
+__device__ __forceinline__ void set_cell(Ray<R> &r, const DSolve<R> &S, const int3 &c, const int4 &A, const int4 &B) {
+#if RC_CHECKED
+    // the cell must lie inside its level or in its halo
+    if (c.x < 0 || c.x > A.z + 1 || c.y < 0 || c.y > A.w + 1 || c.z < 0 || c.z > B.x + 1)
+        RC_IX(-1, 0, SITE_PYRAMID, S);
+#endif
+    const int sj = A.z + 2, sk = sj * (A.w + 2);
+    const bool nx = r.sx < (R)0, ny = r.sy < (R)0, nz = r.sz < (R)0;
+    r.cidx = A.y + c.x + sj * c.y + sk * c.z;
+    r.q = __ldg(S.Pall + RC_IX(r.cidx, S.n_P, SITE_PYRAMID, S));
+    r.fi = A.x + c.x - (int)nx;
+    r.fx = __ldg(S.faces + RC_IX(r.fi, S.n_faces, SITE_FACE, S));
+    r.dx = nx ? -1 : 1;
+    r.dj = ny ? -sj : sj;
+    r.dk = nz ? -sk : sk;
+    r.fj = (float)(c.y - (int)ny);
+    r.fk = (float)(c.z - (int)nz);
+    r.dy = __int_as_float(B.z);
+    r.dz = __int_as_float(B.w);
+}
+
+// Ray state of an emitted bundle.  D: the descriptor in device memory, which
+// holds the run-time Ibmax (S may be its copy in the kernel's parameters).
+template <typename R>
+__device__ __forceinline__ void place_bundle(Ray<R> &r, const DSolve<R> &S, const DSolve<R> &D, const Emitted<R> &e) {
     const int kind = (e.kk >> 16) & 3;
     int ic = e.ij & 0xffff, jc = e.ij >> 16, kc = e.kk & 0xffff;
     // start point: the cell centre, or the wall cell's point on the wall
@@ -437,90 +496,182 @@ __device__ __forceinline__ void place_bundle(Ray<R> &r, const DSolve<R> &S, cons
     r.ratioI = e.ratioI;
     r.invTi4 = e.invTi4;
     const int nb = e.nbg & 0xfffff, g = e.nbg >> 20;
-    r.nb = nb;
-    r.kicol = S.ki + ((size_t)nb * S.nQ + g) * S.nT;
-    r.ic = ic;
-    r.jc = jc;
-    r.kc = kc;
-    r.lev = 0;
-    r.counter = 0;
+    r.kio = (nb * S.nQ + g) * S.nT;
+    r.ln = nb;
+    set_cell(r, S, make_int3(ic, jc, kc), S.lva[0], S.lvb[0]);
+    r.rem = S.lvb[0].y;
     r.tra = (R)1;
     r.De = 0.0;
-    r.Ibmax = kind == 0 ? S.Ibmax_f : kind == 1 ? S.Ibmax_w0 : S.Ibmax_w1;
+    r.dI = (R)0;
+    r.Ibmax = kind == 0 ? D.Ibmax_f : kind == 1 ? D.Ibmax_w0 : D.Ibmax_w1;
     r.tol = kind == 0 ? S.toll : S.tollS;
 }
 
-// Deposit the remaining energy on a black wall emitting Ib_wall
-// (:398-399 and its siblings): De -= Ibmax*tra*(invTi4*e - 1)*ratioI.
-template <typename R>
-__device__ __forceinline__ void wall_deposit(Ray<R> &r, R e) {
-    R c = (r.Ibmax * r.tra) * RT<R>::fma_(r.invTi4, e, (R)-1);
-    c = c * r.ratioI;
-    r.De -= (double)c;
-    r.tra = (R)0;
+// Index of the coarse cell holding fine cell n (1-based): (n + r - 1) / r,
+// as floor(n' m / 2^32) with m = floor(2^32 / r) + 1, exact for n' r < 2^32
+// (the host checks it); m = 0 stands for r = 1.
+__device__ __forceinline__ int coarse_index(int n, int r, unsigned m) {
+    const unsigned np = (unsigned)(n + r - 1);
+    return (int)(m ? __umulhi(np, m) : np);
 }
 
-// Wall condition for wall w at level L (:375-654, with the y/z specular
-// branches reflecting the right component and flag).
+// Integer cell coordinates of a ray on its level (0 and extent + 1: beyond a
+// wall), from the indices of its exit faces.
 template <typename R>
-__device__ __forceinline__ void hit_wall(Ray<R> &r, const DSolve<R> &S, const DLevel<R> &L, int w) {
-    const int t = S.wtype[w];
-    if (t == 1) {  // periodic
-        switch (w) {
-            case RC_WEST: r.ic = L.im; r.xp = S.Lx; break;
-            case RC_EAST: r.ic = 1; r.xp = (R)0; break;
-            case RC_SOUTH: r.jc = L.jm; r.yp = S.Ly; break;
-            case RC_NORTH: r.jc = 1; r.yp = (R)0; break;
-            case RC_BOT: r.kc = L.km; r.zp = S.Lz; break;
-            default: r.kc = 1; r.zp = (R)0; break;
+__device__ __forceinline__ int3 ray_cell(const Ray<R> &r, const int4 &A) {
+    return make_int3(r.fi - A.x + (int)(r.sx < (R)0), (int)r.fj + (int)(r.sy < (R)0), (int)r.fk + (int)(r.sz < (R)0));
+}
+
+// Wall a ray beyond the extents of its level (A, B: its words of lva, lvb)
+// has crossed.
+__device__ __forceinline__ int crossed_wall(const int3 &c, const int4 &A, const int4 &B) {
+    if (c.x == 0) return RC_WEST;
+    if (c.x > A.z) return RC_EAST;
+    if (c.y == 0) return RC_SOUTH;
+    if (c.y > A.w) return RC_NORTH;
+    return c.z == 0 ? RC_BOT : RC_TOP;
+}
+
+// Everything about a ray's next cell that is not the plain move to the
+// neighbour: the wall condition when the cell lies beyond a wall (:375-654,
+// with the y/z specular branches reflecting the right component and flag),
+// the move to coarser levels once the step budget of the level is spent
+// (:210-224), and the faces, offsets and table coordinate of the cell that
+// results.  Returns false when the ray must stop: at a black wall or as a
+// lost ray (the coordinate stays kBlack + wall; retire_ray deposits the rest) or
+// when the budget of the last level is spent.
+template <bool ONE, typename R>
+__device__ __forceinline__ bool enter_cell(Ray<R> &r, const DSolve<R> &S) {
+    int lev = r.ln >> 20;
+    int4 A = load_desc<ONE>(&S.lva[RC_IX(lev, S.nlev, SITE_LEVEL, S)]);
+    int4 B = load_desc<ONE>(&S.lvb[RC_IX(lev, S.nlev, SITE_LEVEL, S)]);
+    int3 c = ray_cell(r, A);
+    const int code = r.q;
+    if (code >= kSpecular) {
+        if (code >= kBlack) return false;
+        const int w = crossed_wall(c, A, B);
+        // periodic: re-enter through the opposite face; specular: stay in
+        // the cell with the crossed component reversed
+        const bool hi = w & 1, per = code == kPeriodic;
+        if (w <= RC_EAST) {
+            r.xp = hi != per ? S.Lx : (R)0;
+            c.x = hi != per ? A.z : 1;
+            if (!per) r.sx = -r.sx, r.isx = -r.isx;
+        } else if (w <= RC_NORTH) {
+            r.yp = hi != per ? S.Ly : (R)0;
+            c.y = hi != per ? A.w : 1;
+            if (!per) r.sy = -r.sy, r.isy = -r.isy;
+        } else {
+            r.zp = hi != per ? S.Lz : (R)0;
+            c.z = hi != per ? B.x : 1;
+            if (!per) r.sz = -r.sz, r.isz = -r.isz;
         }
-    } else if (t == 2) {  // black wall at its own temperature
-        wall_deposit(r, S.Ibw[RC_IX((size_t)w * S.nB + r.nb, 6LL * S.nB, SITE_IBW, S)]);
-    } else if (t == 4 || t == 6) {  // black wall at a field temperature
-        int idx;
-        if (w <= RC_EAST) idx = (r.kc - 1) * L.jm + (r.jc - 1);
-        else if (w <= RC_NORTH) idx = (r.kc - 1) * L.im + (r.ic - 1);
-        else idx = (r.jc - 1) * L.im + (r.ic - 1);
-        const int q = L.Pw[w][RC_IX(idx, w <= RC_EAST ? (long long)L.jm * L.km : (w <= RC_NORTH ? (long long)L.im * L.km
-                                                                                              : (long long)L.im * L.jm),
-                                    SITE_WALL_T, S)];
-        const KIRow<R> row = r.kicol[RC_IX(q >> 8, S.nT, SITE_WALL_ROW, S)];
-        const R fr = coord_frac<R>(q);
-        wall_deposit(r, RT<R>::lerp_(row.ib0, row.ib1, fr));
-    } else if (t == 3) {  // specular
-        switch (w) {
-            case RC_WEST: r.xp = (R)0; r.sx = -r.sx; r.isx = -r.isx; r.ic = 1; break;
-            case RC_EAST: r.xp = S.Lx; r.sx = -r.sx; r.isx = -r.isx; r.ic = L.im; break;
-            case RC_SOUTH: r.yp = (R)0; r.sy = -r.sy; r.isy = -r.isy; r.jc = 1; break;
-            case RC_NORTH: r.yp = S.Ly; r.sy = -r.sy; r.isy = -r.isy; r.jc = L.jm; break;
-            case RC_BOT: r.zp = (R)0; r.sz = -r.sz; r.isz = -r.isz; r.kc = 1; break;
-            default: r.zp = S.Lz; r.sz = -r.sz; r.isz = -r.isz; r.kc = L.km; break;
-        }
-    } else {  // lost ray
-        r.tra = (R)0;
     }
+    while (r.rem <= 0) {
+        if (lev >= S.nlev - 1) {
+            // stopped without a deposit, whatever the transmissivity
+            r.tol = (R)0;
+            r.q = 0;
+            return false;
+        }
+        const DLevel<R> &L = S.lev[lev];
+        c.x = coarse_index(c.x, L.rx, L.mrx);
+        c.y = coarse_index(c.y, L.ry, L.mry);
+        c.z = coarse_index(c.z, L.rz, L.mrz);
+        lev += 1;
+        r.ln += 1 << 20;
+        A = load_desc<ONE>(&S.lva[lev]);
+        B = load_desc<ONE>(&S.lvb[lev]);
+        r.rem = B.y;
+    }
+    set_cell(r, S, c, A, B);
+    return true;
+}
+
+// Re-entry of a ray beyond a periodic wall (coordinate kPeriodic) through the
+// opposite face, with steps left on its level: what enter_cell does for it,
+// without rebuilding what stays.  A channel's rays cross the y and z
+// boundaries in about half of a warp's iterations, one or two lanes at a time.
+template <bool ONE, typename R>
+__device__ __forceinline__ void wrap_cell(Ray<R> &r, const DSolve<R> &S) {
+    const int lev = RC_IX(r.ln >> 20, S.nlev, SITE_LEVEL, S);
+    const int4 A = load_desc<ONE>(&S.lva[lev]);
+    const int km = load_desc<ONE>(&S.lvb[lev]).x;
+    const float fjm = (float)A.w, fkm = (float)km;
+    if (r.fj < 0.f || r.fj > fjm) {
+        const bool hi = r.fj > 0.f;
+        r.yp = hi ? (R)0 : S.Ly;
+        r.fj = hi ? 1.f : fjm - 1.f;
+        r.cidx -= A.w * r.dj;
+    } else if (r.fk < 0.f || r.fk > fkm) {
+        const bool hi = r.fk > 0.f;
+        r.zp = hi ? (R)0 : S.Lz;
+        r.fk = hi ? 1.f : fkm - 1.f;
+        r.cidx -= km * r.dk;
+    } else {
+        const bool hi = r.dx > 0;
+        r.xp = hi ? (R)0 : S.Lx;
+        r.fi = A.x + (hi ? 1 : A.z - 1);
+        r.cidx -= A.z * r.dx;
+        r.fx = __ldg(S.faces + RC_IX(r.fi, S.n_faces, SITE_FACE, S));
+    }
+    r.q = __ldg(S.Pall + RC_IX(r.cidx, S.n_P, SITE_PYRAMID, S));
 }
 
 // Absorption along a path of length ds in a cell of absorption coefficient
-// absco and blackbody intensity blackpow: the step's OERM tally, the
-// transmissivity update and the cutoff deposit (:358-370).
+// absco and blackbody intensity blackpow: the step's OERM tally and the
+// transmissivity update (:358-364).
 template <typename R>
-__device__ __forceinline__ void absorb(Ray<R> &r, R ds, R absco, R blackpow) {
-    const R em = RT<R>::expm1_(-(ds * absco));
+__device__ __forceinline__ void absorb(Ray<R> &r, R ds, R absco, R blackpow, bool go) {
+    // a lane that does not step: nothing absorbed, its last dI kept
+    const R em = go ? RT<R>::expm1_(-(ds * absco)) : (R)0;
     const R alpha = -em;
-    const R dI = RT<R>::fma_(r.invTi4, blackpow, (R)-1);
+    r.dI = go ? RT<R>::fma_(r.invTi4, blackpow, (R)-1) : r.dI;
     R c = r.Ibmax * r.tra;
     c = c * alpha;
     c = c * r.ratioI;
-    c = c * dI;
+    c = c * r.dI;
     r.De -= (double)c;
     r.tra = RT<R>::fma_(r.tra, em, r.tra);
-    if (r.tra < r.tol) {  // cutoff: deposit the rest here (:365-370)
+}
+
+// Last deposit of a ray that has stopped: the rest of its energy in the cell
+// where its transmissivity fell below the cutoff (:365-370), or on the black
+// wall it has reached (:398-399 and its siblings), De -= Ibmax tra ratioI
+// (invTi4 e - 1).  The march retires the stopped rays of a warp together.
+// Returns whether the ray's energy is spent (its transmissivity is then 0).
+template <bool ONE, typename R>
+__device__ __forceinline__ bool retire_ray(Ray<R> &r, const DSolve<R> &S) {
+    if (r.tra < r.tol) {
         R c2 = (r.Ibmax * r.tra) * r.ratioI;
-        c2 = c2 * dI;
+        c2 = c2 * r.dI;
         r.De -= (double)c2;
-        r.tra = (R)0;
+        return true;
     }
+    if (r.q < kBlack) return false;
+    const int w = r.q - kBlack, t = S.wtype[w];
+    R e;
+    if (t == 2) {  // black wall at its own temperature
+        e = S.Ibw[RC_IX((size_t)w * S.nB + (r.ln & 0xfffff), 6LL * S.nB, SITE_IBW, S)];
+    } else if (t == 4 || t == 6) {  // black wall at a field temperature
+        const int lev = RC_IX(r.ln >> 20, S.nlev, SITE_LEVEL, S);
+        const int4 A = load_desc<ONE>(&S.lva[lev]), B = load_desc<ONE>(&S.lvb[lev]);
+        const int im = A.z, jm = A.w, km = B.x;
+        const int3 cell = ray_cell(r, A);
+        const int idx = w <= RC_EAST    ? (cell.z - 1) * jm + (cell.y - 1)
+                        : w <= RC_NORTH ? (cell.z - 1) * im + (cell.x - 1)
+                                        : (cell.y - 1) * im + (cell.x - 1);
+        const long long n = w <= RC_EAST ? (long long)jm * km : w <= RC_NORTH ? (long long)im * km : (long long)im * jm;
+        const int q = S.lev[lev].Pw[w][RC_IX(idx, n, SITE_WALL_T, S)];
+        const KIRow<R> row = S.ki[r.kio + RC_IX(q >> 8, S.nT, SITE_WALL_ROW, S)];
+        e = RT<R>::lerp_(row.ib0, row.ib1, coord_frac<R>(q));
+    } else {
+        return true;  // lost ray
+    }
+    R c = (r.Ibmax * r.tra) * RT<R>::fma_(r.invTi4, e, (R)-1);
+    c = c * r.ratioI;
+    r.De -= (double)c;
+    return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -669,7 +820,17 @@ __device__ __forceinline__ TurnOut<R> scatter_turn_v(R sx, R sy, R sz, int nb, u
 template <typename R>
 __device__ __forceinline__ void scatter_turn(Ray<R> &r, uint4 &ctr, R ks, ScatState<R> &q, const DSolve<R> &S) {
     ctr.w += 1u;
-    const TurnOut<R> o = scatter_turn_v(r.sx, r.sy, r.sz, r.nb, ctr, ks, &S);
+    const TurnOut<R> o = scatter_turn_v(r.sx, r.sy, r.sz, r.ln & 0xfffff, ctr, ks, &S);
+    // the cell stays; its exit faces and neighbours follow the new signs
+    const bool nx = o.sx < (R)0, ny = o.sy < (R)0, nz = o.sz < (R)0;
+    const bool fx = nx != (r.sx < (R)0), fy = ny != (r.sy < (R)0), fz = nz != (r.sz < (R)0);
+    r.fi += fx ? (nx ? -1 : 1) : 0;
+    r.fj += fy ? (ny ? -1.f : 1.f) : 0.f;
+    r.fk += fz ? (nz ? -1.f : 1.f) : 0.f;
+    r.dx = nx ? -1 : 1;
+    r.dj = fy ? -r.dj : r.dj;
+    r.dk = fz ? -r.dk : r.dk;
+    r.fx = __ldg(S.faces + RC_IX(r.fi, S.n_faces, SITE_FACE, S));
     r.sx = o.sx;
     r.sy = o.sy;
     r.sz = o.sz;
@@ -680,119 +841,59 @@ __device__ __forceinline__ void scatter_turn(Ray<R> &r, uint4 &ctr, R ks, ScatSt
 }
 
 // One ray-cell crossing (one iteration of the while loop of march_ray,
-// :252-656).  Returns the step budget (maxs) of the level the step was
-// taken on, which the caller compares with the step counter.  The side of
-// the cell a ray leaves through on each axis follows from the sign of its
-// direction component (never 0: emission floors it at 1e-10).  With SCAT, a
-// bundle whose step is longer than the distance left to its next event
-// stops at the event inside the cell (absorbing along the shortened path),
-// counts the event as a step and sets qs.dist < 0: the caller draws the new
-// direction (scatter_turn) before the next step.  The
-// turn depends neither on the cell nor on the level, so a caller may
-// advance the level first and gather the turns of several lanes into one
-// pass.
+// :252-656) of a ray whose cell lies inside the level (enter_cell).  The side
+// of the cell a ray leaves through on each axis follows from the sign of its
+// direction component (never 0: emission floors it at 1e-10).  The geometry
+// does not depend on the absorption, so the move to the neighbouring cell and
+// the loads of its table coordinate and its new exit face come first; the
+// absorption of this cell covers their latency.  All lanes of a warp run
+// through it together, without a branch; those without `go` keep their ray and
+// load their own cell again.  Returns whether the ray's transmissivity is still above
+// the cutoff.
+// With SCAT, a bundle whose step is longer than the distance left to its next
+// event stops at the event inside the cell (absorbing along the shortened
+// path), counts the event as a step and sets qs.dist < 0: the caller draws the
+// new direction (scatter_turn) before the next step.  The turn depends neither
+// on the cell nor on the level, so a caller may gather the turns of several
+// lanes into one pass.
 template <typename R, bool SCAT>
-__device__ __forceinline__ int march_step(Ray<R> &r, ScatState<R> &qs, const DSolve<R> &S) {
-    // S lives in global memory (read-only during every kernel that steps)
-    const int4 A = __ldg(&S.lva[RC_IX(r.lev, S.nlev, SITE_LEVEL, S)]);
-    const int4 B = __ldg(&S.lvb[RC_IX(r.lev, S.nlev, SITE_LEVEL, S)]);
-    const R fxu = __ldg(S.faces + RC_IX(A.x + r.ic - (int)(r.sx < (R)0), S.n_faces, SITE_FACE, S));
-    const R fyu = __ldg(S.faces + RC_IX(A.y + r.jc - (int)(r.sy < (R)0), S.n_faces, SITE_FACE, S));
-    const R fzu = __ldg(S.faces + RC_IX(A.z + r.kc - (int)(r.sz < (R)0), S.n_faces, SITE_FACE, S));
-#if RC_CHECKED
-    // the cell itself must lie inside its level (a face index alone can be
-    // in the shared faces array while the cell is off its level)
-    if (r.ic < 1 || r.ic > B.x || r.jc < 1 || r.jc > B.y || r.kc < 1 || r.kc > B.z) RC_IX(-1, 0, SITE_PYRAMID, S);
-#endif
-    const int q = __ldg(S.Pall + RC_IX(A.w + cell_index(r.ic, r.jc, r.kc, B.x, B.y), S.n_P, SITE_PYRAMID, S));
-    const KIRow<R> row = load_row(r.kicol + RC_IX(q >> 8, S.nT, SITE_ROW, S));
-    const R dsx = (fxu - r.xp) * r.isx;
-    const R dsy = (fyu - r.yp) * r.isy;
-    const R dsz = (fzu - r.zp) * r.isz;
-    const R a = coord_frac<R>(q);
-    const R absco = RT<R>::lerp_(row.k0, row.k1, a);
-    const R blackpow = RT<R>::lerp_(row.ib0, row.ib1, a);
-    R ds = dsx;
-    if (ds > dsy) ds = dsy;
-    if (ds > dsz) ds = dsz;
+__device__ __forceinline__ bool march_step(Ray<R> &r, ScatState<R> &qs, const DSolve<R> &S, bool go) {
+    KIRow<R> row;
+    load_row_if(go, S.ki + r.kio + RC_IX_IF(go, r.q >> 8, S.nT, SITE_ROW, S), row);
+    const R a = coord_frac<R>(r.q);
+    const R fy = (R)(r.fj * r.dy), fz = (R)(r.fk * r.dz);
+    const R dsx = (r.fx - r.xp) * r.isx;
+    const R dsy = (fy - r.yp) * r.isy;
+    const R dsz = (fz - r.zp) * r.isz;
+    const R ds = RT<R>::fmin_(RT<R>::fmin_(dsx, dsy), dsz);
     // with SCAT, ev: the next scattering event lies inside this cell; the
     // bundle stops there (one absorption path shared with the plain step,
     // so the step loop's code does not grow)
     R dstep = ds;
-    bool ev = false;
+    bool mv = go;
     if constexpr (SCAT) {
-        ev = ds > qs.dist;
-        dstep = ev ? qs.dist : ds;
-        qs.dist = ev ? (R)-1 : qs.dist - ds;
+        const bool ev = ds > qs.dist;
+        dstep = go ? (ev ? qs.dist : ds) : (R)0;
+        qs.dist = go ? (ev ? (R)-1 : qs.dist - ds) : qs.dist;
+        mv = go && !ev;
     }
-    r.xp = (!ev && ds == dsx) ? fxu : RT<R>::fma_(dstep, r.sx, r.xp);
-    r.yp = (!ev && ds == dsy) ? fyu : RT<R>::fma_(dstep, r.sy, r.yp);
-    r.zp = (!ev && ds == dsz) ? fzu : RT<R>::fma_(dstep, r.sz, r.zp);
-    absorb(r, dstep, absco, blackpow);
-    if constexpr (SCAT) {
-        if (ev) {
-            r.counter += 1;
-            return B.w;
-        }
-    }
+    // a lane that does not step needs its position only if it waits for a turn
+    const bool snap = SCAT ? mv : true;
+    r.xp = (snap && ds == dsx) ? r.fx : RT<R>::fma_(dstep, r.sx, r.xp);
+    r.yp = (snap && ds == dsy) ? fy : RT<R>::fma_(dstep, r.sy, r.yp);
+    r.zp = (snap && ds == dsz) ? fz : RT<R>::fma_(dstep, r.sz, r.zp);
     // crossed axis (ties: x only if strictly smallest, :375-377, 524)
-    const int axis = (dsx < dsy) ? ((dsx < dsz) ? 0 : 2) : ((dsy < dsz) ? 1 : 2);
-    const bool ax0 = axis == 0, ax1 = axis == 1;
-    const bool f = ax0 ? (r.sx < (R)0) : (ax1 ? (r.sy < (R)0) : (r.sz < (R)0));
-    const int dlt = f ? -1 : 1;
-    r.ic += ax0 ? dlt : 0;
-    r.jc += ax1 ? dlt : 0;
-    r.kc += (axis == 2) ? dlt : 0;
-    const int nidx = ax0 ? r.ic : (ax1 ? r.jc : r.kc);
-    const int lim = (ax0 ? B.x : (ax1 ? B.y : B.z)) + 1;
-    if (nidx == 0 || nidx == lim) {
-        const int w = 2 * axis + (nidx != 0);
-        if (S.wtype[w] == 1) {
-            // periodic (the common wall of the channel): re-enter through the
-            // opposite face, on a short path of its own
-            const bool hi = nidx != 0;
-            const int ni = hi ? 1 : lim - 1;
-            if (axis == 0) {
-                r.ic = ni;
-                r.xp = hi ? (R)0 : S.Lx;
-            } else if (axis == 1) {
-                r.jc = ni;
-                r.yp = hi ? (R)0 : S.Ly;
-            } else {
-                r.kc = ni;
-                r.zp = hi ? (R)0 : S.Lz;
-            }
-        } else {
-            hit_wall(r, S, S.lev[r.lev], w);
-        }
-    }
-    r.counter += 1;
-    return B.w;
-}
-
-// Index of the coarse cell holding fine cell n (1-based): (n + r - 1) / r,
-// as floor(n' m / 2^32) with m = floor(2^32 / r) + 1, exact for n' r < 2^32
-// (the host checks it); m = 0 stands for r = 1.
-__device__ __forceinline__ int coarse_index(int n, int r, unsigned m) {
-    const unsigned np = (unsigned)(n + r - 1);
-    return (int)(m ? __umulhi(np, m) : np);
-}
-
-// Advance to coarser levels while the step budget of the current level is
-// spent (:210-224).  Returns false when the ray must stop (budget of the
-// last level spent).
-template <typename R>
-__device__ __forceinline__ bool level_advance(Ray<R> &r, const DSolve<R> &S) {
-    while (r.counter >= __ldg(&S.lvb[r.lev]).w) {
-        if (r.lev >= S.nlev - 1) return false;
-        const DLevel<R> &L = S.lev[r.lev];
-        r.ic = coarse_index(r.ic, L.rx, L.mrx);
-        r.jc = coarse_index(r.jc, L.ry, L.mry);
-        r.kc = coarse_index(r.kc, L.rz, L.mrz);
-        r.lev += 1;
-        r.counter = 0;
-    }
-    return true;
+    const bool lt = dsx < dsy, lz = (lt ? dsx : dsy) < dsz;
+    const int mvd = lz ? (lt ? r.dx : r.dj) : r.dk;
+    r.cidx += mv ? mvd : 0;
+    r.fi += mv && lz && lt ? r.dx : 0;
+    r.fj += mv && lz && !lt ? copysignf(1.f, (float)r.sy) : 0.f;
+    r.fk += mv && !lz ? copysignf(1.f, (float)r.sz) : 0.f;
+    r.q = __ldg(S.Pall + RC_IX(r.cidx, S.n_P, SITE_PYRAMID, S));
+    r.fx = __ldg(S.faces + RC_IX(r.fi, S.n_faces, SITE_FACE, S));
+    r.rem -= (int)go;
+    absorb(r, dstep, RT<R>::lerp_(row.k0, row.k1, a), RT<R>::lerp_(row.ib0, row.ib1, a), go);
+    return r.tra > r.tol;
 }
 
 // n / d for a divisor fixed per solve: with M = floor((2^64 - 1)/d) + 1,
@@ -840,6 +941,61 @@ __device__ __forceinline__ ItemId decode_item(const DSolve<R> &S, long long item
         d.k = (int)kw + S.kfirst;
         d.kind = 1 + S.wall_id[(int)slot];
     }
+    return d;
+}
+
+// A tile in flight: its first item, how many of its emitted bundles have not
+// finished, and the first item decoded (0-based i, j, k; q its chunk).  fluid:
+// every item is a cell's, so the others follow from the first by 32-bit
+// arithmetic on small numbers (tile_item).
+struct TileBuf {
+    long long item0;
+    int out, fluid;
+    int i, j, k, v, q, pad;
+};
+
+template <typename R>
+__device__ __forceinline__ void decode_tile(const DSolve<R> &S, long long item0, TileBuf &t) {
+    const ItemId d = decode_item(S, item0);
+    t.item0 = item0;
+    t.out = 0;
+    t.fluid = S.small_div && item0 + kWarp <= S.n_fluid_items;
+    t.i = d.i - 1;
+    t.j = d.j - 1;
+    t.k = d.k;
+    t.v = d.v;
+    t.q = d.h0 / S.rpt;
+}
+
+// n / d for n < 2^16, d <= 2^15 with m = magic32(d): exact (n d < 2^32).
+__device__ __forceinline__ int sdiv(int n, unsigned m) { return m ? (int)__umulhi((unsigned)n, m) : n; }
+
+// Item it (0..31) of a tile.  The chunks of one (cell, replicate) are a power
+// of two up to 32, or a multiple of 32: a tile starts at the first chunk of a
+// (cell, replicate), or holds one only.
+template <typename R>
+__device__ __forceinline__ ItemId tile_item(const DSolve<R> &S, const TileBuf &t, int it) {
+    if (!t.fluid) return decode_item(S, t.item0 + it);
+    ItemId d;
+    d.kind = 0;
+    d.h0 = (t.q + (it & (S.gsize - 1))) * S.rpt;
+    d.v = t.v;
+    int i = t.i, j = t.j, k = t.k;
+    if (S.gsize < kWarp) {
+        const int x = t.v + (it >> (__ffs(S.gsize) - 1));
+        const int c = sdiv(x, S.m_nvar);
+        d.v = x - c * S.nVar;
+        i += c;
+        const int ci = sdiv(i, S.m_imax);
+        i -= ci * S.imax;
+        j += ci;
+        const int cj = sdiv(j, S.m_jmax);
+        j -= cj * S.jmax;
+        k += cj;
+    }
+    d.i = i + 1;
+    d.j = j + 1;
+    d.k = k;
     return d;
 }
 

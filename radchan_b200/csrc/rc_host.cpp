@@ -638,6 +638,8 @@ void build_grid_level(const rc_params &p, int level, GridLevel &g) {
 
     const float dy = p.Ly * 1.0f / jm;  // definitions.h:85-86
     const float dz = p.Lz * 1.0f / km;
+    g.dy = dy;
+    g.dz = dz;
     for (int i = 0; i < jm + 1; i++) g.yu[i] = i * dy;
     for (int i = 0; i < km + 1; i++) g.zu[i] = i * dz;
     g.y[0] = -dy / 2;

@@ -34,6 +34,7 @@ enum WallType : int {
 // One multigrid level (definitions.h:60-136).
 struct GridLevel {
     int im = 0, jm = 0, km = 0, maxs = 0;
+    float dy = 0.f, dz = 0.f;       // yu[j] = j dy, zu[k] = k dz (one rounding each)
     std::vector<float> xu, yu, zu;  // faces: im+1, jm+1, km+1
     std::vector<float> x, y, z;     // centres with ghosts: im+2, jm+2, km+2
 };

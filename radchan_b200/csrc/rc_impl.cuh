@@ -371,6 +371,12 @@ struct Impl : ImplBase {
         return RC_OK;
     }
 
+    // Table coordinates of a level with its halo.
+    long long level_cells(int l) const {
+        const rc_params &p = c->p;
+        return (long long)(p.maxi[l] + 2) * (p.maxj[l] + 2) * (p.maxk[l] + 2);
+    }
+
     int init(int nslots) {
         std::string *err_ = &c->err;
         const rc_params &p = c->p;
@@ -381,7 +387,9 @@ struct Impl : ImplBase {
         face_off.assign(nl, 0);
         lev_off.assign(nl, 0);
         {
-            std::vector<float> faces;
+            // one element before and after: a ray beyond a wall has its exit
+            // face one past the wall's
+            std::vector<float> faces(1, 0.f);
             long long po = 0;
             for (int l = 0; l < nl; ++l) {
                 const GridLevel &g = c->grid[l];
@@ -390,9 +398,10 @@ struct Impl : ImplBase {
                 faces.insert(faces.end(), g.yu.begin(), g.yu.end());
                 faces.insert(faces.end(), g.zu.begin(), g.zu.end());
                 lev_off[l] = (int)po;
-                po += (long long)p.maxi[l] * p.maxj[l] * p.maxk[l];
+                po += level_cells(l);
                 if (po > 0x7fffffffLL) return set_err(err_, RC_E_INVALID, "grid too large for 32-bit level offsets");
             }
+            faces.push_back(0.f);
             n_faces = (long long)faces.size();
             n_pyramid = po;
             int rc = upload(d_faces, faces, err_);
@@ -447,14 +456,13 @@ struct Impl : ImplBase {
             // multigrid pyramid and wall emission arrays
             s.d_levT.assign(nl, nullptr);
             {
-                long long tot = 0;
-                for (int l = 0; l < nl; ++l) tot += (long long)p.maxi[l] * p.maxj[l] * p.maxk[l];
-                RC_CK(cudaMalloc((void **)&s.d_levAll, tot * sizeof(uint16_t)));
-                RC_CK(cudaMemset(s.d_levAll, 0, tot * sizeof(uint16_t)));
+                RC_CK(cudaMalloc((void **)&s.d_levAll, n_pyramid * sizeof(uint16_t)));
+                RC_CK(cudaMemset(s.d_levAll, 0, n_pyramid * sizeof(uint16_t)));
                 for (int l = 0; l < nl; ++l) s.d_levT[l] = s.d_levAll + lev_off[l];
             }
             LevelJobs &J = s.jobs;
             memset(&J, 0, sizeof(J));
+            for (int w = 0; w < 6; ++w) J.halo[w] = halo_code(c->wt[w], w);
             auto add_job = [&](void *dst, int type, int l, int face, long long n) {
                 LevelJob &jb = J.job[J.njobs++];
                 jb.dst = dst;
@@ -471,8 +479,7 @@ struct Impl : ImplBase {
                 J.total += n;
             };
             for (int l = 0; l < nl; ++l) {
-                const long long n = (long long)p.maxi[l] * p.maxj[l] * p.maxk[l];
-                add_job(s.d_levT[l], 0, l, 0, n);
+                add_job(s.d_levT[l], 0, l, 0, level_cells(l));
                 for (int w = 0; w < 6; ++w) {
                     const int t = c->wt[w];
                     if (t != WT_BLACK_CELL && t != WT_BLACK_FACE) continue;
@@ -510,12 +517,12 @@ struct Impl : ImplBase {
         RC_CK(cudaGetDeviceProperties(&prop, c->device));
         c->num_sms = prop.multiProcessorCount;
         smem_opt_in = (int)prop.sharedMemPerBlockOptin;
-        RC_CK(cudaFuncSetAttribute(k_march<R, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_opt_in));
-        RC_CK(cudaFuncSetAttribute(k_march<R, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_opt_in));
-        RC_CK(cudaFuncSetAttribute(k_march<R, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_opt_in));
-        RC_CK(cudaFuncSetAttribute(k_march<R, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_opt_in));
-        RC_CK(cudaFuncSetAttribute(k_march<R, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_opt_in));
-        RC_CK(cudaFuncSetAttribute(k_march<R, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_opt_in));
+        for (int v = 0; v < 6; ++v) {
+            RC_CK(cudaFuncSetAttribute(march_fn<false>(2 + v / 2, v & 1), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       smem_opt_in));
+            RC_CK(cudaFuncSetAttribute(march_fn<true>(2 + v / 2, v & 1), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       smem_opt_in));
+        }
         if (p.grey) return set_grey_tables();
         return RC_OK;
     }
@@ -730,9 +737,13 @@ struct Impl : ImplBase {
             L.yu = d_yu[l];
             L.zu = d_zu[l];
             L.P = s.d_levT[l];
-            d.lva[l] = make_int4(face_off[l], face_off[l] + L.im + 1, face_off[l] + L.im + 1 + L.jm + 1, lev_off[l]);
-            d.lvb[l] = make_int4(L.im, L.jm, L.km, L.maxs);
+            int dy, dz;
+            memcpy(&dy, &c->grid[l].dy, 4);
+            memcpy(&dz, &c->grid[l].dz, 4);
+            d.lva[l] = make_int4(face_off[l], lev_off[l], L.im, L.jm);
+            d.lvb[l] = make_int4(L.km, L.maxs, dy, dz);
             for (int w = 0; w < 6; ++w) L.Pw[w] = s.d_lw[l][w];
+            d.steps_to[l] = (l ? d.steps_to[l - 1] : 0) + p.maxs[l];
         }
         d.imax = p.imax;
         d.jmax = p.jmax;
@@ -800,6 +811,10 @@ struct Impl : ImplBase {
         d.mg_imax = magic(p.imax);
         d.mg_jmax = magic(p.jmax);
         d.mg_nwc = magic(d.nwc);
+        d.m_nvar = magic32(p.nVar);
+        d.m_imax = magic32(p.imax);
+        d.m_jmax = magic32(p.jmax);
+        d.small_div = std::max(p.nVar, std::max(p.imax, p.jmax)) <= 32768;
     }
 
     // Multiply-high reciprocal of a divisor d (see fdiv): floor((2^64-1)/d)+1,
@@ -878,12 +893,15 @@ struct Impl : ImplBase {
     }
 
     size_t march_smem(int block, int rpt_max, bool scat = false) const {
-        return scat ? march_smem_bytes<R, true>(block, rpt_max) : march_smem_bytes<R, false>(block, rpt_max);
+        const int nbuf = tile_bufs(rpt_max);
+        return scat ? march_smem_bytes<R, true>(block, rpt_max, nbuf) : march_smem_bytes<R, false>(block, rpt_max, nbuf);
     }
 
-    static void (*march_fn(int minb, bool scat))(MarchArgs) {
-        if (scat) return minb <= 2 ? k_march<R, 2, true> : minb == 3 ? k_march<R, 3, true> : k_march<R, 4, true>;
-        return minb <= 2 ? k_march<R, 2, false> : minb == 3 ? k_march<R, 3, false> : k_march<R, 4, false>;
+    template <bool ONE>
+    static void (*march_fn(int minb, bool scat))(MarchParams<R, ONE>) {
+        if (scat)
+            return minb <= 2 ? k_march<R, 2, true, ONE> : minb == 3 ? k_march<R, 3, true, ONE> : k_march<R, 4, true, ONE>;
+        return minb <= 2 ? k_march<R, 2, false, ONE> : minb == 3 ? k_march<R, 3, false, ONE> : k_march<R, 4, false, ONE>;
     }
 
     // Long-ray priority list of a one-solve launch (k_prio_kmin +
@@ -948,23 +966,14 @@ struct Impl : ImplBase {
 
     // scat: < 0 takes this context's medium (scattering tables set or not);
     // a launch over several contexts passes whether any of them scatters.
+    // one: the host copy of the descriptor when the launch marches one solve.
     int launch_march(const DSolve<R> *d_solves, const long long *d_tiles, int nsolves, long long total_tiles,
                      unsigned long long *d_counter, int block, int rpt_max, cudaStream_t st, int minb = 0,
-                     const Slot<R> *prio = nullptr, int scat = -1) {
+                     const Slot<R> *prio = nullptr, int scat = -1, const DSolve<R> *one = nullptr) {
         std::string *err_ = &c->err;
         RC_FAILPOINT("march");
         if (minb <= 0) minb = c->minb;
         const bool sc = scat < 0 ? nA > 0 : scat > 0;
-        auto fn = march_fn(minb, sc);
-        const size_t smem = march_smem(block, rpt_max, sc);
-        if ((int)smem > smem_opt_in) return set_err(err_, RC_E_INVALID, "rays_per_thread too large for shared memory");
-        int per_sm = 0;
-        RC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem));
-        per_sm = std::max(per_sm, 1);
-        const long long warps_needed = total_tiles;
-        long long grid = std::min<long long>((long long)per_sm * c->num_sms, (warps_needed + block / kWarp - 1) / (block / kWarp));
-        grid = std::max<long long>(grid, 1);
-        RC_CK(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st));
         MarchArgs a;
         a.solves = d_solves;
         a.tile_start = d_tiles;
@@ -972,10 +981,31 @@ struct Impl : ImplBase {
         a.total_tiles = total_tiles;
         a.tile_counter = d_counter;
         a.rpt_max = rpt_max;
+        a.nbuf = tile_bufs(rpt_max);
         a.prio_tiles = prio ? prio->d_prio : nullptr;
         a.tile_prio = prio ? prio->d_tprio : nullptr;
         a.n_prio = prio ? prio->d_nprio : nullptr;
-        fn<<<(unsigned)grid, block, smem, st>>>(a);
+        if (one) {
+            MarchParams<R, true> m;
+            m.m = a;
+            m.one = *one;
+            return launch_march_fn(march_fn<true>(minb, sc), m, block, march_smem(block, rpt_max, sc), st);
+        }
+        MarchParams<R, false> m;
+        m.m = a;
+        return launch_march_fn(march_fn<false>(minb, sc), m, block, march_smem(block, rpt_max, sc), st);
+    }
+    template <typename F, typename P>
+    int launch_march_fn(F fn, const P &m, int block, size_t smem, cudaStream_t st) {
+        std::string *err_ = &c->err;
+        if ((int)smem > smem_opt_in) return set_err(err_, RC_E_INVALID, "rays_per_thread too large for shared memory");
+        int per_sm = 0;
+        RC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem));
+        per_sm = std::max(per_sm, 1);
+        const long long blocks = (m.m.total_tiles + block / kWarp - 1) / (block / kWarp);
+        const long long grid = std::max<long long>(1, std::min<long long>((long long)per_sm * c->num_sms, blocks));
+        RC_CK(cudaMemsetAsync(m.m.tile_counter, 0, sizeof(unsigned long long), st));
+        fn<<<(unsigned)grid, block, smem, st>>>(m);
         RC_CK(cudaGetLastError());
         return RC_OK;
     }
@@ -1114,7 +1144,7 @@ struct Impl : ImplBase {
         rc = enqueue_prio(s, s.st, prio);
         if (rc) return rc;
         rc = launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, c->block, rpt, s.st, 0,
-                          prio ? &s : nullptr);
+                          prio ? &s : nullptr, -1, s.h_desc);
         if (rc) return rc;
         RC_CK(cudaEventRecord(s.e_march1, s.st));
         rc = launch_tally(s.d_desc, s.d_out, 1, tally_cells(), s.st);
@@ -1149,7 +1179,7 @@ struct Impl : ImplBase {
             rc = enqueue_prio(s, s.st, prio);
             if (rc) return rc;
             rc = launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, block, rpt, s.st, minb,
-                              prio ? &s : nullptr);
+                              prio ? &s : nullptr, -1, s.h_desc);
             if (rc) return rc;
             RC_CK(cudaEventRecord(s.e_march1, s.st));
             RC_CK(cudaEventSynchronize(s.e_march1));

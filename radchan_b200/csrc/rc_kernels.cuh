@@ -245,6 +245,7 @@ constexpr int kMaxJobs = RC_MAX_LEVELS * 7 + 2;
 struct LevelJobs {
     LevelJob job[kMaxJobs];
     int njobs;
+    int halo[6];  // code of the cells beyond each wall (halo_code)
     long long total;
 };
 
@@ -262,15 +263,26 @@ __global__ void k_levels(const float *__restrict__ T, int imax, int jmax, int km
         uint16_t *dst = (uint16_t *)J.dst;
         const float rxf = (float)J.rx, ryf = (float)J.ry, rzf = (float)J.rz;
         if (J.type == 0) {
-            const int ic = (int)(l % J.im) + 1;
-            const long long r = l / J.im;
-            const int jc = (int)(r % J.jm) + 1;
-            const int kc = (int)(r / J.jm) + 1;
+            // every cell with its halo; the halo's edges belong to no ray
+            const int ic = (int)(l % (J.im + 2));
+            const long long r = l / (J.im + 2);
+            const int jc = (int)(r % (J.jm + 2));
+            const int kc = (int)(r / (J.jm + 2));
+            const int w = ic == 0       ? RC_WEST
+                          : ic > J.im   ? RC_EAST
+                          : jc == 0     ? RC_SOUTH
+                          : jc > J.jm   ? RC_NORTH
+                          : kc == 0     ? RC_BOT
+                          : kc > J.km   ? RC_TOP
+                                        : -1;
+            if (w >= 0) {
+                dst[l] = (uint16_t)jobs.halo[w];
+                continue;
+            }
             const float t1 = ((float)ic - 0.5f) * rxf + 1.0f;
             const float t2 = ((float)jc - 0.5f) * ryf + 1.0f;
             const float t3 = ((float)kc - 0.5f) * rzf + 1.0f;
-            dst[cell_index(ic, jc, kc, J.im, J.jm)] =
-                (uint16_t)table_coord((R)tex_sample(T, nx, ny, nz, t1, t2, t3), T0, inv_dT, nT);
+            dst[l] = (uint16_t)table_coord((R)tex_sample(T, nx, ny, nz, t1, t2, t3), T0, inv_dT, nT);
         } else {
             const int w = J.type - 1;
             float x, y, z;
@@ -315,7 +327,7 @@ __global__ void k_trace(const DSolve<R> *Sp, int n, const rc_bundle_id *ids, rc_
     rec.tra = 0.f;
     rec.De = 0.0;
     Emitted<R> e;
-    const bool ok = emit_bundle(e, S, id.kind, id.i, id.j, id.k, id.v, id.h);
+    const bool ok = emit_bundle(e, S, S.row, id.kind, id.i, id.j, id.k, id.v, id.h);
     rec.nb = e.nbg & 0xfffff;
     rec.g = e.nbg >> 20;
     rec.sx = (float)e.sx;
@@ -326,31 +338,36 @@ __global__ void k_trace(const DSolve<R> *Sp, int n, const rc_bundle_id *ids, rc_
         ScatState<R> qs;
         uint4 ctr = make_uint4(0u, 0u, 0u, 0u);
         R ks = (R)0;
-        place_bundle(r, S, e);
+        place_bundle(r, S, S, e);
         if (SCAT) {
             ctr = scatter_counter(S.imax, S.jmax, id.kind, id.i, id.j, id.k, id.v, id.h, 0u);
             ks = scatter_coef(S, e.nbg & 0xfffff, e.nbg >> 20);
             qs.dist = scatter_first_dist(ks > (R)0 ? scatter_first_lnu(S, ctr) : (R)0, ks);
         }
-        bool active = level_advance(r, S);
         int ns = 0;
+        bool active = true;
         while (active) {
-            if (ns < max_cells && cells) {
-                int *c = cells + ((size_t)t * max_cells + ns) * 4;
-                c[0] = r.lev;
-                c[1] = r.ic;
-                c[2] = r.jc;
-                c[3] = r.kc;
+            if (r.q >= kSpecular || r.rem <= 0) {
+                if (r.q == kPeriodic && r.rem > 0) wrap_cell<false>(r, S);
+                else active = enter_cell<false>(r, S);
             }
-            march_step<R, SCAT>(r, qs, S);
-            if (SCAT && qs.dist < (R)0) scatter_turn(r, ctr, ks, qs, S);
+            if (!active || r.q >= kSpecular) continue;
+            if (ns < max_cells && cells) {
+                const int3 cc = ray_cell(r, S.lva[r.ln >> 20]);
+                int *c = cells + ((size_t)t * max_cells + ns) * 4;
+                c[0] = r.ln >> 20;
+                c[1] = cc.x;
+                c[2] = cc.y;
+                c[3] = cc.z;
+            }
+            active = march_step<R, SCAT>(r, qs, S, true);
+            if (SCAT && active && qs.dist < (R)0) scatter_turn(r, ctr, ks, qs, S);
             ns++;
-            active = r.tra > r.tol;
-            if (active) active = level_advance(r, S);
         }
+        const bool spent = retire_ray<false>(r, S);
         rec.nsteps = ns;
-        rec.end_level = r.lev;
-        rec.tra = (float)r.tra;
+        rec.end_level = r.ln >> 20;
+        rec.tra = spent ? 0.f : (float)r.tra;
         rec.De = r.De;
     }
     out[t] = rec;
@@ -365,7 +382,7 @@ __global__ void k_sample_bands(const DSolve<R> *Sp, int kind, int n, const float
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     int b, q;
-    select_band_g(*Sp, kind, (R)u_b[t], (R)u_g[t], b, q);
+    select_band_g(*Sp, Sp->row, kind, (R)u_b[t], (R)u_g[t], b, q);
     nb[t] = b;
     g[t] = q;
 }

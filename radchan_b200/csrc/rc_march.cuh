@@ -15,21 +15,21 @@ namespace rc {
 //   * bundles are emitted in converged waves of 32 (all lanes decode their
 //     item and run the Philox draws, direction, band/g search and OERM
 //     weights together) into a per-warp ring in shared memory whenever the
-//     ring holds fewer than 32 bundles;
+//     ring holds fewer than kRefill bundles;
 //   * every lane traces one ray; the warp steps all its rays until at least
-//     kFeedIdle lanes are idle, then hands those lanes the next emitted
-//     bundles (warp ballot + prefix count);
-//   * two tiles can be in flight: once every bundle of a tile has been
+//     kFeedIdle lanes are idle, then retires the rays that stopped and hands
+//     those lanes the next emitted bundles (warp ballot + prefix count);
+//   * two to four tiles can be in flight (tile_bufs): once every bundle of a tile has been
 //     emitted, the warp fetches the next tile (of the same solve) and keeps
-//     emitting from it while the last rays of the previous tile finish, so
-//     long rays do not leave the other lanes idle at tile ends;
+//     emitting from it while the last rays of earlier tiles finish, so long
+//     rays do not leave the other lanes idle;
 //   * each bundle's FP64 tally goes to its own shared-memory slot; when a
 //     tile's last bundle has finished, its slots are summed in bundle
 //     order, so the result does not depend on which lane traced which
 //     bundle.
-// Shared memory per warp is the ring (64 emitted bundles of 32 bytes: the
+// Shared memory per warp is the ring (42 emitted bundles of 32 bytes: the
 // start position is rebuilt from the emitting cell when a lane takes the
-// bundle) and two slot arrays; everything else stays in L1-cached global
+// bundle) and the slot arrays; everything else stays in L1-cached global
 // memory, so that most of the SM's 256 KB of L1/shared storage caches the
 // temperature pyramid and the k / I_b tables (48-byte entries, an earlier
 // layout, were 1.2% slower; 64-byte entries 4%).  The scattering variant
@@ -42,12 +42,26 @@ struct MarchArgs {
     long long total_tiles;
     unsigned long long *tile_counter;
     int rpt_max;
+    int nbuf;  // tiles a warp has in flight (tile_bufs)
     // long-ray priority (one solve only; NULL: tiles in natural order): the
     // first *n_prio claims take prio_tiles[], the rest take the natural
     // order and skip the tiles whose tile_prio byte is set
     const unsigned *prio_tiles;
     const unsigned char *tile_prio;
     const unsigned *n_prio;
+};
+// A launch over one solve carries its descriptor in the kernel's parameters:
+// what the march reads of it then comes from constant memory (operands and
+// uniform registers) instead of loads through L1 into registers.  The run-time
+// values (Ibmax, table row) are still read from the copy in device memory.
+template <typename R, bool ONE>
+struct MarchParams {
+    MarchArgs m;
+};
+template <typename R>
+struct MarchParams<R, true> {
+    MarchArgs m;
+    DSolve<R> one;
 };
 
 // Long-ray priority list.  A bundle whose path is long -- nearly parallel
@@ -106,7 +120,7 @@ __global__ void k_prio_tiles(const DSolve<R> *Sp, float thr, const float *kmin, 
                 const float Lw = dx / fmaxf(fabsf(sx), 1e-10f);
                 if (!(Lw > Lthr)) continue;
                 int nb, g;
-                select_band_g(S, it.kind, (R)rc_u01(d.z), (R)rc_u01(d.w), nb, g);
+                select_band_g(S, S.row, it.kind, (R)rc_u01(d.z), (R)rc_u01(d.w), nb, g);
                 const float k = kmin[nb * S.nQ + g];
                 cand = k * Lthr < tau;  // ln(1/tol) / k > Lthr
             }
@@ -122,6 +136,7 @@ __global__ void k_prio_tiles(const DSolve<R> *Sp, float thr, const float *kmin, 
 template <typename R, bool SCAT>
 struct WarpShared {
     Emitted<R> ring[kRing];
+    TileBuf tile[kTileBufs];
 };
 // With scattering, also the free path to the first event of every ring
 // entry (drawn by the emission wave), and the scattering coefficient and
@@ -131,6 +146,7 @@ struct WarpShared {
 template <typename R>
 struct WarpShared<R, true> {
     Emitted<R> ring[kRing];
+    TileBuf tile[kTileBufs];
     R dist[kRing];
     R ks[kWarp];
     uint32_t nev[kWarp];
@@ -161,28 +177,39 @@ __device__ __forceinline__ void flush_counters(DScalars *sc, unsigned long long 
     nsteps = nbund = 0;
 }
 
+template <bool ONE, typename R>
+__device__ __forceinline__ const DSolve<R> &one_or(const MarchParams<R, ONE> &prm, const DSolve<R> &D) {
+    if constexpr (ONE) return prm.one;
+    else return D;
+}
+
+// Ring position of a running index (below 2 kRing).
+__device__ __forceinline__ int ring_at(int i) { return i < kRing ? i : i - kRing; }
+
 // MINB: resident 256-thread blocks per SM the register allocation must
 // allow (2: up to 128 registers, 3: 80, 4: 64).  SCAT: the variant for
 // media with scattering particles (solves without them run in it unchanged).
-template <typename R, int MINB, bool SCAT>
-__global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
+template <typename R, int MINB, bool SCAT, bool ONE>
+__global__ void __launch_bounds__(256, MINB) k_march(const __grid_constant__ MarchParams<R, ONE> prm) {
+    const MarchArgs &a = prm.m;
     extern __shared__ __align__(16) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    // volatile: kept in a register instead of read again at every use
+    int lane, warp;
+    asm volatile("mov.u32 %0, %%laneid;" : "=r"(lane));
+    asm volatile("mov.u32 %0, %1;" : "=r"(warp) : "r"(threadIdx.x >> 5));
+    const int nwarps = blockDim.x >> 5;
     WarpShared<R, SCAT> *ws = reinterpret_cast<WarpShared<R, SCAT> *>(smem) + warp;
     const size_t wbytes = ((sizeof(WarpShared<R, SCAT>) * nwarps) + 15) & ~(size_t)15;
     const int pool_max = kWarp * a.rpt_max;
-    double *slots0 = reinterpret_cast<double *>(smem + wbytes) + (size_t)warp * 2 * pool_max;
+    double *slots0 = reinterpret_cast<double *>(smem + wbytes) + (size_t)warp * a.nbuf * pool_max;
     const DSolve<R> *solves = reinterpret_cast<const DSolve<R> *>(a.solves);
     const unsigned lt = (1u << lane) - 1u;
     const DSolve<R> *Sp = solves;
 
     // warp-uniform state
     int cur_solve = -1;
-    long long item0_0 = 0, item0_1 = 0;  // first item of the tile in each buffer
     unsigned busy = 0u;     // bit p: buffer p holds a tile not yet reduced
-    unsigned emitted = 0u;  // bit p: every bundle of buffer p's tile emitted
-    int out0 = 0, out1 = 0; // emitted bundles of each buffer not finished yet
-    int epar = -1;          // buffer being emitted from
+    int epar = -1;          // buffer being emitted from (-1: every bundle of the busy buffers is emitted)
     int next_b = 0, head = 0, count = 0;
     bool drained = false;   // no more tiles
     unsigned long long pending = ~0ull;  // fetched tile waiting for a solve switch
@@ -193,21 +220,20 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
     const unsigned long long nprio = a.n_prio ? (unsigned long long)__ldg(a.n_prio) : 0ull;
     const unsigned long long total = (unsigned long long)a.total_tiles + nprio;
     const unsigned long long all_warps = (unsigned long long)gridDim.x * nwarps;
-    // lanes tracing a ray, and lanes whose ray belongs to buffer 1
-    // (warp-uniform; kept in step with the lanes' own flags)
-    unsigned amask = 0u, p1mask = 0u;
+    unsigned amask = 0u;    // lanes tracing a ray (warp-uniform; kept in step with the lanes' own flags)
     // lane state
     bool active = false;
-    int myslot = 0;  // slot of the lane's bundle: parity * pool_max + index
+    int myslot = 0;  // the lane's bundle: buffer << 12 | index in the tile
     unsigned long long nsteps = 0, nbund = 0;
-    Ray<R> r;
+    Ray<R> r = {};
     ScatState<R> qs;
+    qs.dist = (R)0;
 
     for (;;) {
         // ---- fetch the next tile into a free buffer
-        if (!drained && (epar < 0 || ((emitted >> epar) & 1u))) {
-            const int fpar = (epar < 0) ? 0 : (epar ^ 1);
-            if (!((busy >> fpar) & 1u)) {
+        if (epar < 0 && !drained) {
+            const int fpar = __ffs(~busy) - 1;
+            if (fpar < a.nbuf) {
                 unsigned long long tile = pending;
                 if (tile == ~0ull) {
                     // ends: every pass advances chunk_next or the shared
@@ -249,9 +275,9 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
                     drained = true;
                     pending = ~0ull;
                 } else {
-                    const int so = solve_of_tile(a.tile_start, a.nsolves, tile);
+                    const int so = ONE ? 0 : solve_of_tile(a.tile_start, a.nsolves, tile);
                     if (so != cur_solve && busy) {
-                        pending = tile;  // switch solves only once both buffers are reduced
+                        pending = tile;  // switch solves only once every buffer is reduced
                     } else {
                         pending = ~0ull;
                         if (so != cur_solve) {
@@ -259,16 +285,11 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
                             Sp = solves + so;
                             cur_solve = so;
                         }
-                        const long long i0 =
-                            ((long long)(tile - (unsigned long long)a.tile_start[so]) + Sp->tile_base) * kWarp;
-                        if (fpar) item0_1 = i0;
-                        else item0_0 = i0;
+                        const long long t0 = (long long)(ONE ? tile : tile - (unsigned long long)a.tile_start[so]);
+                        if (lane == 0) decode_tile(one_or<ONE>(prm, *Sp), (t0 + Sp->tile_base) * kWarp, ws->tile[fpar]);
                         double *sl = slots0 + fpar * pool_max;
                         for (int b = lane; b < kWarp * Sp->rpt; b += kWarp) sl[b] = 0.0;
                         busy |= 1u << fpar;
-                        emitted &= ~(1u << fpar);
-                        if (fpar) out1 = 0;
-                        else out0 = 0;
                         epar = fpar;
                         next_b = 0;
                         __syncwarp();
@@ -276,45 +297,46 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
                 }
             }
         }
-        const DSolve<R> &S = *Sp;
+        const DSolve<R> &D = *Sp;  // with the run-time values
+        const DSolve<R> &S = one_or<ONE>(prm, D);
         const int rpt = S.rpt;
         const int lrpt = __ffs(rpt) - 1;  // rpt is a power of two
         const int pool = kWarp * rpt;
         // ---- converged emission wave: one bundle per lane
-        if (count < kWarp && epar >= 0 && !((emitted >> epar) & 1u)) {
+        if (count < kRefill && epar >= 0) {
             const int b = next_b + lane;
             Emitted<R> e;
             R dist0 = (R)kNoEvent;
-            bool ok = false;
-            if (b < pool) {
-                const ItemId it = decode_item(S, (epar ? item0_1 : item0_0) + (b >> lrpt));
-                const int h = it.h0 + (b & (rpt - 1));
-                if (it.kind >= 0 && h < S.photmax) {
-                    nbund++;
-                    // with particles, draw 1 (scatter_first_lnu, written
-                    // out: the call form spilled) before the emission
-                    // itself: little is live then, so the variant fits the
-                    // register budget without spilling
-                    R lnu = (R)0;
-                    if constexpr (SCAT) {
-                        if (S.nA > 0) {
-                            const uint4 c0 = scatter_counter(S.imax, S.jmax, it.kind, it.i, it.j, it.k, it.v, h, 0u);
-                            rc_u32x4 c;
-                            c.x = c0.x;
-                            c.y = c0.y;
-                            c.z = c0.z;
-                            c.w = 1u;
-                            const rc_u32x4 d = rc_philox4x32_10(c, S.key0, S.key1);
-                            lnu = -RT<R>::log_((R)rc_u01(d.x));
-                        }
-                    }
-                    ok = emit_bundle(e, S, it.kind, it.i, it.j, it.k, it.v, h);
-                    e.kk |= (b << 18) | (epar << 29);
-                    if constexpr (SCAT) {
-                        const R ks = scatter_coef(S, e.nbg & 0xfffff, e.nbg >> 20);
-                        if (ks > (R)0) dist0 = lnu / ks;  // scatter_first_dist
-                    }
+            ItemId it = tile_item(S, ws->tile[epar], b >> lrpt);
+            int h = it.h0 + (b & (rpt - 1));
+            const bool valid = it.kind >= 0 && h < S.photmax;
+            if (!valid) {  // a padding item: emit anything, and drop it
+                it.kind = 0;
+                it.i = it.j = it.k = 1;
+                it.v = h = 0;
+            }
+            nbund += valid;
+            // with particles, draw 1 (scatter_first_lnu, written out: the
+            // call form spilled) before the emission itself: little is live
+            // then, so the variant fits the register budget without spilling
+            R lnu = (R)0;
+            if constexpr (SCAT) {
+                if (S.nA > 0) {
+                    const uint4 c0 = scatter_counter(S.imax, S.jmax, it.kind, it.i, it.j, it.k, it.v, h, 0u);
+                    rc_u32x4 c;
+                    c.x = c0.x;
+                    c.y = c0.y;
+                    c.z = c0.z;
+                    c.w = 1u;
+                    const rc_u32x4 d = rc_philox4x32_10(c, S.key0, S.key1);
+                    lnu = -RT<R>::log_((R)rc_u01(d.x));
                 }
+            }
+            const bool ok = emit_bundle(e, S, D.row, it.kind, it.i, it.j, it.k, it.v, h) && valid;
+            e.kk |= (b << 18) | (epar << 29);
+            if constexpr (SCAT) {
+                const R ks = scatter_coef(S, e.nbg & 0xfffff, e.nbg >> 20);
+                if (ks > (R)0) dist0 = lnu / ks;  // scatter_first_dist
             }
             const unsigned m = __ballot_sync(0xffffffffu, ok);
             int pos = __popc(m & lt);
@@ -327,7 +349,7 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
                 unsigned key = 0xffffffffu;
                 if (ok) {
                     const int nb = e.nbg & 0xfffff, g = e.nbg >> 20;
-                    key = __float_as_uint((float)S.ki[RC_IX(((size_t)nb * S.nQ + g) * S.nT + S.row,
+                    key = __float_as_uint((float)S.ki[RC_IX(((size_t)nb * S.nQ + g) * S.nT + D.row,
                                                             (long long)S.nB * S.nQ * S.nT, SITE_EMIT_ROW, S)]
                                               .k0);  // k >= 0: monotone bits
                 }
@@ -339,83 +361,67 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
                 pos = rank;
             }
             if (ok) {
-                ws->ring[(head + count + pos) & (kRing - 1)] = e;
-                if constexpr (SCAT) ws->dist[(head + count + pos) & (kRing - 1)] = dist0;
+                const int at = ring_at(head + count + pos);
+                ws->ring[at] = e;
+                if constexpr (SCAT) ws->dist[at] = dist0;
             }
             count += __popc(m);
-            if (epar) out1 += __popc(m);
-            else out0 += __popc(m);
+            if (lane == 0) ws->tile[epar].out += __popc(m);
             next_b += kWarp;
-            if (next_b >= pool) emitted |= 1u << epar;
+            if (next_b >= pool) epar = -1;
             __syncwarp();
         }
         // ---- idle lanes take emitted bundles
         {
-            const unsigned m = ~amask;
-            const int navail = min(count, __popc(m));
-            bool took = false, fin = false;
-            if (!active) {
-                const int rank = __popc(m & lt);
-                if (rank < navail) {
-                    const Emitted<R> &e = ws->ring[(head + rank) & (kRing - 1)];
-                    place_bundle(r, S, e);
+            const int navail = min(count, kWarp - __popc(amask));
+            if (navail > 0) {
+                const int rank = __popc(~amask & lt);
+                const bool take = !active && rank < navail;
+                if (take) {
+                    const int at = ring_at(head + rank);
+                    const Emitted<R> &e = ws->ring[at];
+                    place_bundle(r, S, D, e);
                     if constexpr (SCAT) {
-                        qs.dist = ws->dist[(head + rank) & (kRing - 1)];
+                        qs.dist = ws->dist[at];
                         ws->ks[lane] = scatter_coef(S, e.nbg & 0xfffff, e.nbg >> 20);
                         ws->nev[lane] = 0u;
                     }
-                    myslot = ((e.kk >> 29) & 1) * pool_max + ((e.kk >> 18) & 0x7ff);
-                    took = true;
-                    active = level_advance(r, S);
-                    if (!active) {
-                        slots0[myslot] = r.De;
-                        fin = true;
-                    }
+                    myslot = (((e.kk >> 29) & 3) << 12) | ((e.kk >> 18) & 0x7ff);
+                    active = true;
                 }
+                head = ring_at(head + navail);
+                count -= navail;
+                amask |= __ballot_sync(0xffffffffu, take);
+                __syncwarp();
             }
-            head = (head + navail) & (kRing - 1);
-            count -= navail;
-            if (navail > 0) {
-                const unsigned tk = __ballot_sync(0xffffffffu, took);
-                const unsigned t1 = __ballot_sync(0xffffffffu, took && myslot >= pool_max);
-                const unsigned fi = __ballot_sync(0xffffffffu, fin);
-                p1mask = (p1mask & ~tk) | t1;
-                amask = (amask | tk) & ~fi;
-                out1 -= __popc(fi & t1);
-                out0 -= __popc(fi & ~t1);
-            }
-            __syncwarp();
         }
         // ---- step every active ray; stay in this loop until enough lanes
-        //      are idle to be worth handing out bundles (or a tile can be
-        //      reduced, or every lane is idle)
+        //      are idle to be worth handing out bundles (or, with nothing to
+        //      hand out, a tile can be reduced, or every lane is idle)
+        bool check;
         {
-            const bool can_feed =
-                count > 0 || (epar >= 0 && !((emitted >> epar) & 1u)) ||
-                (!drained && (epar < 0 || (((emitted >> epar) & 1u) && !((busy >> (epar ^ 1)) & 1u))));
+            const bool can_feed = count > 0 || epar >= 0 || (!drained && busy != (1u << a.nbuf) - 1u);
+            // leave the loop once this few lanes move, or (nothing to hand
+            // out) as soon as a ray stops
+            const int enough = can_feed ? kWarp - kFeedIdle : 0;
+            const unsigned on_stop = can_feed ? 0u : 0xffffffffu;
+            unsigned am = amask;
             for (;;) {
-                bool fin = false;
+                // a black wall ends the ray; other walls, a spent step
+                // budget and a cell to be rebuilt take the slow path
+                active = active && r.q < kBlack;
+                bool go = active;
+                if constexpr (SCAT) go = active && !(qs.dist < (R)0);
+                if (go && (r.q >= kSpecular || r.rem <= 0)) {
+                    if (r.q == kPeriodic && r.rem > 0) wrap_cell<ONE>(r, S);
+                    else active = enter_cell<ONE>(r, S);
+                }
+                go = go && active && r.q < kSpecular;
+                const bool above = march_step<R, SCAT>(r, qs, S, go);
+                active = active && (above || !go);
                 bool wait_turn = false;
                 if constexpr (SCAT) wait_turn = active && qs.dist < (R)0;
-                if (active && !wait_turn) {
-                    const int budget = march_step<R, SCAT>(r, qs, S);
-                    nsteps++;
-                    bool done = !(r.tra > r.tol);
-                    if (!done && r.counter >= budget) done = !level_advance(r, S);
-                    if (done) {
-                        slots0[myslot] = r.De;
-                        active = false;
-                        fin = true;
-                    }
-                    if constexpr (SCAT) wait_turn = active && qs.dist < (R)0;
-                }
-                const unsigned fm = __ballot_sync(0xffffffffu, fin);
-                if (fm) {
-                    const int n1 = __popc(fm & p1mask);
-                    out1 -= n1;
-                    out0 -= __popc(fm) - n1;
-                    amask &= ~fm;
-                }
+                am = __ballot_sync(0xffffffffu, active);
                 // lanes stopped at a scattering event wait for a turn pass,
                 // which draws all their new directions at once; the pass is
                 // long and runs on the waiting lanes only, so it waits until
@@ -424,13 +430,27 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
                 bool turn_now = false;
                 if constexpr (SCAT) {
                     tm = __ballot_sync(0xffffffffu, wait_turn);
-                    turn_now = __popc(tm) >= kTurnGather || (tm && !(amask & ~tm));
+                    turn_now = __popc(tm) >= kTurnGather || (tm && !(am & ~tm));
                 }
-                const int nidle = kWarp - __popc(amask & ~tm);
-                if (nidle == kWarp) break;
-                if (nidle >= kFeedIdle && (can_feed || turn_now)) break;
-                if (fm && ((((busy & emitted) & 1u) && out0 == 0) || (((busy & emitted) & 2u) && out1 == 0))) break;
+                const unsigned moving = am & ~tm;
+                if (__popc(moving) <= enough || ((am ^ amask) & on_stop) || (SCAT && turn_now && __popc(moving) <= kWarp - kFeedIdle))
+                    break;
             }
+            // ---- retire the rays that stopped: last deposit, tally slot
+            bool last = false;
+            if (am != amask) {
+                if (((amask & ~am) >> lane) & 1u) {
+                    retire_ray<ONE>(r, S);
+                    nsteps += S.steps_to[r.ln >> 20] - r.rem;
+                    slots0[(myslot >> 12) * pool_max + (myslot & 0xfff)] = r.De;
+                    last = atomicSub(&ws->tile[myslot >> 12].out, 1) == 1;
+                }
+                amask = am;
+                __syncwarp();  // (without it ptxas keeps the warp's state in vector registers)
+            }
+            // a tile may be complete: its last ray has stopped, or its last
+            // wave was empty
+            check = __any_sync(0xffffffffu, last) || count == 0;
         }
         // ---- scattering: the new directions of every lane stopped at an
         //      event, once kTurnGather lanes wait or no traced ray is left
@@ -439,8 +459,8 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
             const unsigned tw = __ballot_sync(0xffffffffu, active && qs.dist < (R)0);
             const bool turn_now = __popc(tw) >= kTurnGather || (tw && !(amask & ~tw));
             if (turn_now && active && qs.dist < (R)0) {
-                const int mypar = myslot >= pool_max, myb = myslot - mypar * pool_max;
-                const ItemId it = decode_item(S, (mypar ? item0_1 : item0_0) + (myb >> lrpt));
+                const int myb = myslot & 0xfff;
+                const ItemId it = tile_item(S, ws->tile[myslot >> 12], myb >> lrpt);
                 uint4 c = scatter_counter(S.imax, S.jmax, it.kind, it.i, it.j, it.k, it.v, it.h0 + (myb & (rpt - 1)),
                                           ws->nev[lane]);
                 scatter_turn(r, c, ws->ks[lane], qs, S);
@@ -449,22 +469,23 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
         }
         // ---- reduce finished tiles: chunk sums in bundle order, group sums
         //      in item order
-#pragma unroll
-        for (int par = 0; par < 2; ++par) {
-            const int outp = par ? out1 : out0;
-            if (((busy & emitted) >> par) & 1u && outp == 0) {
-                __syncwarp();
+        if (check) {
+            __syncwarp();
+            unsigned ready = busy & (epar < 0 ? ~0u : ~(1u << epar));
+            ready &= __ballot_sync(0xffffffffu, ws->tile[lane < kTileBufs ? lane : 0].out == 0);
+            const int lgs = __ffs(S.gsize) - 1;  // items of a group: a power of two
+            while (ready) {
+                const int par = __ffs(ready) - 1;
+                ready &= ready - 1u;
                 const double *sl = slots0 + par * pool_max;
                 double s = 0.0;
                 for (int h = 0; h < rpt; ++h) s += sl[lane * rpt + h];
-                const int gs = S.gsize;
-                const int base = (lane / gs) * gs;
+                const int base = lane >> lgs << lgs;
                 double g = 0.0;
-                for (int q = 0; q < gs; ++q) g += __shfl_sync(0xffffffffu, s, base + q);
-                const long long item = (par ? item0_1 : item0_0) + lane;
-                if (lane == base && item < S.n_items) S.partial[RC_IX(item / gs, S.n_partial, SITE_PARTIAL, S)] = g;
+                for (int q = 0; q < S.gsize; ++q) g += __shfl_sync(0xffffffffu, s, base + q);
+                const long long item = ws->tile[par].item0 + lane;
+                if (lane == base && item < S.n_items) S.partial[RC_IX(item >> lgs, S.n_partial, SITE_PARTIAL, S)] = g;
                 busy &= ~(1u << par);
-                if (epar == par) epar = -1;
                 __syncwarp();
             }
         }
@@ -473,10 +494,14 @@ __global__ void __launch_bounds__(256, MINB) k_march(MarchArgs a) {
     if (cur_solve >= 0) flush_counters(Sp->sc, nsteps, nbund, lane);
 }
 
+// Tiles a warp keeps in flight.  A tile's slots are held until its longest
+// ray has finished, and with every buffer held the warp runs out of bundles.
+constexpr int tile_bufs(int rpt_max) { return rpt_max <= 4 ? kTileBufs : 2; }
+
 template <typename R, bool SCAT>
-constexpr size_t march_smem_bytes(int block, int rpt_max) {
+constexpr size_t march_smem_bytes(int block, int rpt_max, int nbuf) {
     return ((((size_t)sizeof(WarpShared<R, SCAT>) * (block / kWarp)) + 15) & ~(size_t)15) +
-           (size_t)(block / kWarp) * 2 * kWarp * rpt_max * sizeof(double);
+           (size_t)(block / kWarp) * nbuf * kWarp * rpt_max * sizeof(double);
 }
 
 }  // namespace rc

@@ -182,11 +182,11 @@ int rc_create(const rc_params *p, int device, rc_ctx **out) {
     for (int l = 0; l < p->grid_num; ++l) build_grid_level(*p, l, c->grid[l]);
     c->dbl = p->floatpoint == 1;
     // measured best on B200 for the 64^3 narrow-band and 32^3 grey channels:
-    // 4 bundles per work item, 256-thread blocks, 64-register budget (FP32);
-    // the FP64 ray state needs the larger register budget
+    // 4 bundles per work item; FP32 72 registers and 128-thread blocks, seven
+    // of which fit an SM; the FP64 ray state needs the larger budget
     c->rpt = 4;
-    c->block = 256;
-    c->minb = c->dbl ? 2 : 4;
+    c->block = c->dbl ? 256 : 128;
+    c->minb = c->dbl ? 2 : 3;
     int rc;
     if (c->dbl) {
         auto *im = new Impl<double>();
@@ -874,7 +874,7 @@ int solve_noalloc_t(rc_ctx *c, const float *T_dev, int zstart, double *q64, doub
     const size_t wall_bytes = 2 * (size_t)s.h_desc->nwc * sizeof(double);
     if (nwalls < 2 && qw64) RC_CK(cudaMemsetAsync(qw64, 0, wall_bytes, st));
     if (nwalls < 2 && vw64) RC_CK(cudaMemsetAsync(vw64, 0, wall_bytes, st));
-    rc = im.launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, c->block, rpt, st);
+    rc = im.launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, c->block, rpt, st, 0, nullptr, -1, s.h_desc);
     if (rc) return rc;
     rc = im.launch_tally(s.d_desc, s.d_out, 1, im.tally_cells(), st);
     if (rc) return rc;
