@@ -950,8 +950,8 @@ struct Impl : ImplBase {
             RC_CK(cudaMalloc((void **)&s.d_kmin, nbq * sizeof(float)));
             s.kmin_cap = nbq;
         }
-        if (!s.d_nprio) RC_CK(cudaMalloc((void **)&s.d_nprio, sizeof(unsigned)));
-        RC_CK(cudaMemsetAsync(s.d_nprio, 0, sizeof(unsigned), st));
+        if (!s.d_nprio) RC_CK(cudaMalloc((void **)&s.d_nprio, 2 * sizeof(unsigned)));
+        RC_CK(cudaMemsetAsync(s.d_nprio, 0, 2 * sizeof(unsigned), st));
         k_prio_kmin<R><<<(nbq + 255) / 256, 256, 0, st>>>(s.d_desc, s.d_kmin);
         RC_CK(cudaGetLastError());
         const long long grid = std::max<long long>(1, std::min<long long>((nt + 7) / 8, (long long)c->num_sms * 16));

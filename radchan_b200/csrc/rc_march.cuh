@@ -44,8 +44,9 @@ struct MarchArgs {
     int rpt_max;
     int nbuf;  // tiles a warp has in flight (tile_bufs)
     // long-ray priority (one solve only; NULL: tiles in natural order): the
-    // first *n_prio claims take prio_tiles[], the rest take the natural
-    // order and skip the tiles whose tile_prio byte is set
+    // first n_prio[0] claims take the head of prio_tiles[], the next
+    // n_prio[1] its end (backwards), the rest take the natural order and skip
+    // the tiles whose tile_prio byte is set
     const unsigned *prio_tiles;
     const unsigned char *tile_prio;
     const unsigned *n_prio;
@@ -74,10 +75,16 @@ struct MarchParams<R, true> {
 // d_x the distance from its start to the x wall it moves towards, k_min the
 // smallest absorption coefficient of its band and g point over the table
 // rows the field's temperatures span (k_prio_kmin); a tile is listed when
-// some bundle has L > thr * Lx.  The draws are the emission's own (Philox
+// some bundle has L > thr * Lx, and in the first part of the list when
+// L > kSoloPath * thr * Lx.  Such a ray decides when a short launch ends: a
+// warp that has claimed its tile claims no other before its rays have
+// finished, so the ray is not held up by the emission and feeding of others
+// (its warp then steps it 2-3 times as often).  The draws are the emission's own (Philox
 // counter of the bundle, select_band_g), so the estimate sees the same
 // direction, band and g point the march will trace.  Only the order in
 // which tiles are claimed changes, never a result.
+constexpr float kSoloPath = 16.f;
+
 template <typename R>
 __global__ void k_prio_kmin(const DSolve<R> *Sp, float *kmin) {
     const DSolve<R> &S = *Sp;
@@ -103,7 +110,7 @@ __global__ void k_prio_tiles(const DSolve<R> *Sp, float thr, const float *kmin, 
     for (long long tile = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); tile < S.n_tiles;
          tile += nw) {
         const ItemId it = decode_item(S, tile * kWarp + lane);
-        bool cand = false;
+        bool cand = false, solo = false;
         if (it.kind >= 0) {
             const uint32_t cell = (it.kind == 0)
                                       ? (uint32_t)((it.i - 1) + S.imax * ((it.j - 1) + S.jmax * (it.k - 1)))
@@ -111,7 +118,7 @@ __global__ void k_prio_tiles(const DSolve<R> *Sp, float thr, const float *kmin, 
             const float x0 = it.kind == 0 ? (float)S.xc[it.i] : (it.kind == 1 ? 0.f : Lx);
             const float tau = it.kind == 0 ? tau_f : tau_w;
             const int h1 = min(it.h0 + S.rpt, S.photmax);
-            for (int h = it.h0; h < h1 && !cand; ++h) {
+            for (int h = it.h0; h < h1 && !solo; ++h) {
                 const rc_u32x4 d = bundle_draws(S.key0, S.key1, h, it.v, it.kind, cell);
                 const float u = rc_u01(d.y);
                 // s_x as emit_bundle draws it: 1 - 2u (fluid), sqrt(1 - u) / -sqrt(u) (walls)
@@ -122,13 +129,15 @@ __global__ void k_prio_tiles(const DSolve<R> *Sp, float thr, const float *kmin, 
                 int nb, g;
                 select_band_g(S, S.row, it.kind, (R)rc_u01(d.z), (R)rc_u01(d.w), nb, g);
                 const float k = kmin[nb * S.nQ + g];
-                cand = k * Lthr < tau;  // ln(1/tol) / k > Lthr
+                cand = cand || k * Lthr < tau;  // ln(1/tol) / k > Lthr
+                solo = Lw > kSoloPath * Lthr && k * (kSoloPath * Lthr) < tau;
             }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, cand);
+        const unsigned m = __ballot_sync(0xffffffffu, cand), ms = __ballot_sync(0xffffffffu, solo);
         if (lane == 0) {
             tile_prio[tile] = m != 0u;
-            if (m) prio_tiles[atomicAdd(n_prio, 1u)] = (unsigned)tile;
+            if (ms) prio_tiles[atomicAdd(n_prio, 1u)] = (unsigned)tile;
+            else if (m) prio_tiles[S.n_tiles - 1 - atomicAdd(n_prio + 1, 1u)] = (unsigned)tile;
         }
     }
 }
@@ -189,8 +198,12 @@ __device__ __forceinline__ int ring_at(int i) { return i < kRing ? i : i - kRing
 // MINB: resident 256-thread blocks per SM the register allocation must
 // allow (2: up to 128 registers, 3: 80, 4: 64).  SCAT: the variant for
 // media with scattering particles (solves without them run in it unchanged).
+// Registers of the variants (MINB, the occupancy knob): 64 lets four 256-thread
+// blocks onto an SM, 72 seven 128-thread blocks, 128 two 256-thread blocks.
+constexpr int march_regs(int minb) { return minb >= 4 ? 64 : minb == 3 ? 72 : 128; }
+
 template <typename R, int MINB, bool SCAT, bool ONE>
-__global__ void __launch_bounds__(256, MINB) k_march(const __grid_constant__ MarchParams<R, ONE> prm) {
+__global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(const __grid_constant__ MarchParams<R, ONE> prm) {
     const MarchArgs &a = prm.m;
     extern __shared__ __align__(16) unsigned char smem[];
     // volatile: kept in a register instead of read again at every use
@@ -213,13 +226,10 @@ __global__ void __launch_bounds__(256, MINB) k_march(const __grid_constant__ Mar
     int next_b = 0, head = 0, count = 0;
     bool drained = false;   // no more tiles
     unsigned long long pending = ~0ull;  // fetched tile waiting for a solve switch
-    // tiles claimed from the queue but not started: [chunk_next, chunk_end)
-    unsigned long long chunk_next = 0, chunk_end = 0;
-    // with the long-ray priority list, the claim space is the listed tiles
-    // followed by all tiles in natural order (listed ones skipped there)
-    const unsigned long long nprio = a.n_prio ? (unsigned long long)__ldg(a.n_prio) : 0ull;
-    const unsigned long long total = (unsigned long long)a.total_tiles + nprio;
-    const unsigned long long all_warps = (unsigned long long)gridDim.x * nwarps;
+    // tiles claimed from the queue but not started: chunk_left from chunk_next on
+    unsigned long long chunk_next = 0;
+    int chunk_left = 0;
+    bool hold = false;      // a tile of the priority list's first part is in flight: claim no other
     unsigned amask = 0u;    // lanes tracing a ray (warp-uniform; kept in step with the lanes' own flags)
     // lane state
     bool active = false;
@@ -231,37 +241,46 @@ __global__ void __launch_bounds__(256, MINB) k_march(const __grid_constant__ Mar
 
     for (;;) {
         // ---- fetch the next tile into a free buffer
-        if (epar < 0 && !drained) {
+        if (epar < 0 && !drained && !hold) {
             const int fpar = __ffs(~busy) - 1;
             if (fpar < a.nbuf) {
-                unsigned long long tile = pending;
+                // with the long-ray priority list, the claim space is the
+                // listed tiles followed by all tiles in natural order (listed
+                // ones skipped there); the counts are read here, not kept
+                const volatile unsigned *np = a.n_prio;
+                const unsigned nsolo = np ? np[0] : 0u, nprio = np ? nsolo + np[1] : 0u;
+                const unsigned long long total = (unsigned long long)a.total_tiles + nprio;
+                unsigned long long tile = ONE ? ~0ull : pending;
                 if (tile == ~0ull) {
                     // ends: every pass advances chunk_next or the shared
                     // counter, and a claim at or past `total` ends the queue
                     for (;;) {
-                        if (chunk_next >= chunk_end) {
+                        if (chunk_left <= 0) {
                             // guided self-scheduling: claim up to kChunkMax
                             // consecutive tiles (usually of one solve), so a
-                            // warp keeps two tiles of the same solve in
+                            // warp keeps its tiles of the same solve in
                             // flight; claim fewer as the queue drains to keep
-                            // the tail short
-                            unsigned long long c0 = 0;
+                            // the tail short, and the longest rays one by one
                             if (lane == 0) {
                                 const unsigned long long seen = *(volatile unsigned long long *)a.tile_counter;
                                 const unsigned long long rem = seen < total ? total - seen : 0ull;
-                                const unsigned long long k =
-                                    max(1ull, min((unsigned long long)kChunkMax, rem / (4ull * all_warps)));
-                                c0 = atomicAdd(a.tile_counter, k);
-                                chunk_end = min(c0 + k, total);
+                                const unsigned long long k = rem / (4ull * gridDim.x * nwarps);
+                                chunk_left = seen < nsolo ? 1 : (int)max(1ull, min((unsigned long long)kChunkMax, k));
+                                chunk_next = atomicAdd(a.tile_counter, (unsigned long long)chunk_left);
                             }
-                            c0 = __shfl_sync(0xffffffffu, c0, 0);
-                            chunk_end = __shfl_sync(0xffffffffu, chunk_end, 0);
-                            chunk_next = c0;
+                            chunk_next = __shfl_sync(0xffffffffu, chunk_next, 0);
+                            chunk_left = __shfl_sync(0xffffffffu, chunk_left, 0);
                         }
-                        tile = chunk_next < chunk_end ? chunk_next++ : total;
-                        if (!a.n_prio || tile >= total) break;
+                        tile = chunk_next++;
+                        chunk_left--;
+                        if (tile >= total) {
+                            tile = total;
+                            break;
+                        }
+                        if (!np) break;
                         if (tile < nprio) {
-                            tile = __ldg(a.prio_tiles + tile);
+                            hold = tile < nsolo;
+                            tile = __ldg(a.prio_tiles + (hold ? tile : (unsigned long long)a.total_tiles - 1 - (tile - nsolo)));
                             break;
                         }
                         if (!__ldg(a.tile_prio + (tile - nprio))) {
@@ -400,7 +419,7 @@ __global__ void __launch_bounds__(256, MINB) k_march(const __grid_constant__ Mar
         //      hand out, a tile can be reduced, or every lane is idle)
         bool check;
         {
-            const bool can_feed = count > 0 || epar >= 0 || (!drained && busy != (1u << a.nbuf) - 1u);
+            const bool can_feed = count > 0 || epar >= 0 || (!drained && !hold && busy != (1u << a.nbuf) - 1u);
             // leave the loop once this few lanes move, or (nothing to hand
             // out) as soon as a ray stops
             const int enough = can_feed ? kWarp - kFeedIdle : 0;
@@ -488,6 +507,7 @@ __global__ void __launch_bounds__(256, MINB) k_march(const __grid_constant__ Mar
                 busy &= ~(1u << par);
                 __syncwarp();
             }
+            if (!busy) hold = false;
         }
         if (drained && !busy) break;
     }
