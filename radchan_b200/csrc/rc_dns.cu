@@ -34,19 +34,59 @@ struct DnsArgs {
     double *Qnew, *Varnew, *Knew, *Gnew;  // (0:imax+1, jn, kloc)
     unsigned long long *n_clamped;
     double stefan, Tin, Tin4, Height, underrelax;
+    double r_stefan, r_Tin4, r_Height;  // reciprocals, rounded to nearest (div_by)
+    int recip;                          // the three divisors and all quotients lie well inside the normal range
     int imax, jmax, kloc, jstart, jn, west, east;
     int nT, dT;
     unsigned long long Mnx, Mjn, MdT;  // fdiv multipliers of imax+2, jn, dT
+    unsigned mnx, mjn, mdT;            // their 32-bit forms (mdT: 0 unless 2 <= dT < 65536)
+    int small;                         // 32-bit indices suffice
     double Tnb[RC_DNS_MAX_T], kP[RC_DNS_MAX_T], slope[RC_DNS_MAX_T];
 };
 
+// x / c, correctly rounded, for a divisor c known beforehand with its rounded
+// reciprocal y = RN(1/c): a quotient within one ulp, its exact remainder by a
+// fused multiply-add, and one correction (P. W. Markstein, IBM J. Res. Dev.
+// 34, 1990: the corrected quotient is the rounded one when y is the rounded
+// reciprocal).  The first correction brings x y within the one ulp that the
+// theorem asks for.  For finite x with every value in the normal range; a zero
+// quotient keeps its sign by the first product alone.
+__device__ __forceinline__ double div_by(double x, double c, double y) {
+    const double q0 = x * y;
+    const double q = fma(fma(-q0, c, x), y, q0);
+    return x == 0.0 ? q0 : fma(fma(-q, c, x), y, q);
+}
+
+// (double)v / stefan / Tin4 (and / Height), each division rounded.
+__device__ __forceinline__ double scaled(const DnsArgs &a, float v, bool wall) {
+    if (a.recip && fabsf(v) <= 3.4028235e38f) {  // finite
+        double q = div_by(div_by((double)v, a.stefan, a.r_stefan), a.Tin4, a.r_Tin4);
+        if (wall) q = div_by(q, a.Height, a.r_Height);
+        return q;
+    }
+    double q = (double)v / a.stefan / a.Tin4;
+    if (wall) q = q / a.Height;
+    return q;
+}
+
+// n / d by a multiply-high with the divisor's reciprocal: 64 bits (fdiv), or
+// 32 bits with m = floor(2^32 / d) + 1 (0 for d = 1), exact for n d < 2^32.
+__device__ __forceinline__ unsigned long long quot(unsigned long long n, unsigned long long M, unsigned) {
+    return fdiv(n, M);
+}
+__device__ __forceinline__ unsigned quot(unsigned n, unsigned long long, unsigned m) { return m ? __umulhi(n, m) : n; }
+
 // One thread per output cell (grid-stride), i fastest, so every load and
 // store of a warp is contiguous; (i, j, k) and linear_int's row come from
-// exact multiply-high divisions (fdiv) instead of integer division.  The
-// kernel is bound by instruction issue: the five IEEE double divisions the
-// Fortran's statement order requires take most of its ~245 instructions per
-// cell (measured on B200; 6 resident blocks per SM were 2-3% faster than 4,
-// two cells per thread no faster).
+// exact multiply-high divisions instead of integer division, in 32 bits (I)
+// when the pencil is small enough (dns_args: cells times its longer edge
+// below 2^32; the 192x128x128 pencil is at a seventh of that).  The kernel is
+// bound by instruction issue and, behind it, DRAM: with 64-bit indices and
+// five plain divisions it took 335 instructions per cell and 40.3 us for
+// 192x128x128 (153 MB); with div_by and 64-bit indices 36.7 us; in 32 bits
+// and with zero values kept off the plain division 188 instructions and
+// 31.0 us, 4.9 TB/s.
+template <typename I>
 __global__ void __launch_bounds__(256, 6) k_dns_source(const __grid_constant__ DnsArgs a) {
     __shared__ double sT[RC_DNS_MAX_T], sK[RC_DNS_MAX_T], sS[RC_DNS_MAX_T];
     for (int t = threadIdx.x; t < a.nT; t += blockDim.x) {
@@ -55,40 +95,34 @@ __global__ void __launch_bounds__(256, 6) k_dns_source(const __grid_constant__ D
         sS[t] = a.slope[t];
     }
     __syncthreads();
-    const int nx = a.imax + 2;
-    const unsigned long long n = (unsigned long long)nx * a.jn * a.kloc;
+    const I nx = a.imax + 2;
+    const I n = nx * (I)a.jn * (I)a.kloc;
     unsigned int clamped = 0;
-    for (unsigned long long c = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; c < n;
-         c += (unsigned long long)gridDim.x * blockDim.x) {
-        const unsigned long long r = fdiv(c, a.Mnx);  // (j, k) row
-        const int i = (int)(c - r * nx);
-        const unsigned long long k0 = fdiv(r, a.Mjn);
-        const int jl = (int)(r - k0 * a.jn) + 1;  // 1..jn, local to the pencil
-        const int kl = (int)k0 + 1;               // 1..kloc
-        const int jg = a.jstart + jl - 1;         // 1..jmax, the solve's j
-        const long long wcell = (long long)(kl - 1) * a.jmax + (jg - 1);
+    for (I c = blockIdx.x * (I)blockDim.x + threadIdx.x; c < n; c += (I)gridDim.x * blockDim.x) {
+        const I r = quot(c, a.Mnx, a.mnx);  // (j, k) row
+        const I i = c - r * nx;
+        const I k0 = quot(r, a.Mjn, a.mjn);  // 0..kloc-1
+        const I j0 = r - k0 * (I)a.jn;       // 0..jn-1, local to the pencil
+        const I wcell = k0 * (I)a.jmax + (I)(a.jstart - 1) + j0;  // the solve's (j, k) row
         const bool wall = (i == 0) || (i == nx - 1);
+        // the cell's or the wall's values, by one pair of loads; get_results_
+        // writes 0 on a wall whose flux is not computed
+        const I at = wall ? (i == 0 ? (I)0 : (I)a.jmax * (I)a.kloc) + wcell : wcell * (I)a.imax + (i - 1);
         float q = 0.f, s = 0.f;
-        if (wall) {
-            // get_results_ writes 0 on a wall whose flux is not computed
-            if (i == 0 ? a.west : a.east) {
-                const long long w = (i == 0 ? 0LL : (long long)a.jmax * a.kloc) + wcell;
-                q = __ldg(a.Wq + w);
-                s = __ldg(a.Ws + w);
-            }
-        } else {
-            q = __ldg(a.Qc + (wcell * a.imax + (i - 1)));
-            s = __ldg(a.Sc + (wcell * a.imax + (i - 1)));
+        if (!wall || (i == 0 ? a.west : a.east)) {
+            q = __ldg((wall ? a.Wq : a.Qc) + at);
+            s = __ldg((wall ? a.Ws : a.Sc) + at);
         }
-        const double T1 = __ldg(a.T1 + (i + (long long)nx * (jl + (long long)(a.jn + 2) * kl)));
-        double Qn = (double)q / a.stefan / a.Tin4;
-        if (wall) Qn = Qn / a.Height;
-        const double Vn = (double)s / a.stefan / a.Tin4;
+        const double T1 = __ldg(a.T1 + (i + nx * (j0 + 1 + (I)(a.jn + 2) * (k0 + 1))));
+        double Qn = scaled(a, q, wall);
+        const double Vn = scaled(a, s, false);
         const double x0 = T1 * a.Tin;
         const double d = x0 - sT[0];
         // t = int(x0 - x(1)) / int(x(2) - x(1)): both truncate toward zero
         int t;
-        if (d > -2147483648.0 && d < 2147483648.0) {
+        if (d > -1.0 && d < 65536.0 && a.mdT) {
+            t = (int)__umulhi((unsigned)(int)d, a.mdT);
+        } else if (d > -2147483648.0 && d < 2147483648.0) {
             const int ti = (int)d;
             const int tq = (int)fdiv((unsigned long long)(ti < 0 ? -(long long)ti : ti), a.MdT);
             t = ti < 0 ? -tq : tq;
@@ -138,6 +172,11 @@ int dns_args(const rc_ctx *c, const rc_dns_coupling *cfg, DnsArgs &a, std::strin
     a.Tin4 = pow(cfg->Tin, 4.0);
     a.Height = cfg->Height;
     a.underrelax = cfg->underrelax;
+    a.r_stefan = 1.0 / a.stefan;
+    a.r_Tin4 = 1.0 / a.Tin4;
+    a.r_Height = 1.0 / a.Height;
+    auto mid = [](double v) { return fabs(v) > 0x1p-200 && fabs(v) < 0x1p200; };
+    a.recip = mid(a.stefan) && mid(a.Tin4) && mid(a.Height);
     a.imax = p.imax;
     a.jmax = p.jmax;
     a.kloc = c->kloc;
@@ -150,6 +189,13 @@ int dns_args(const rc_ctx *c, const rc_dns_coupling *cfg, DnsArgs &a, std::strin
     a.Mnx = Impl<float>::magic((unsigned long long)(p.imax + 2));
     a.Mjn = Impl<float>::magic((unsigned long long)a.jn);
     a.MdT = Impl<float>::magic((unsigned long long)a.dT);
+    a.mnx = Impl<float>::magic32((unsigned)(p.imax + 2));
+    a.mjn = Impl<float>::magic32((unsigned)a.jn);
+    a.mdT = a.dT < 65536 ? Impl<float>::magic32((unsigned)a.dT) : 0u;
+    // every index and division: cells of the padded pencil and of the solve's
+    // planes times the longer divisor (and one grid stride beyond the end)
+    const double cells = (double)(p.imax + 2) * std::max(p.jmax, a.jn + 2) * (c->kloc + 2);
+    a.small = cells * std::max(p.imax + 2, a.jn) < 4.0e9;
     for (int t = 0; t < cfg->nTemp; ++t) {
         a.Tnb[t] = cfg->Tnb[t];
         a.kP[t] = cfg->kP[t];
@@ -171,14 +217,11 @@ int launch_dns(const rc_ctx *c, const DnsArgs &a, cudaStream_t st, std::string *
     RC_FAILPOINT("dns");
     // every block resident at once: the SMs' worth of blocks, at most one
     // cell per thread
-    static int per_sm = 0;
-    if (!per_sm) {
-        RC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_dns_source, 256, 0));
-        per_sm = std::max(per_sm, 1);
-    }
+    constexpr int per_sm = 6;  // the kernel's launch bounds
+    auto fn = a.small ? k_dns_source<unsigned> : k_dns_source<unsigned long long>;
     const long long n = (long long)(a.imax + 2) * a.jn * a.kloc;
     const int grid = (int)std::max<long long>(1, std::min<long long>((n + 255) / 256, (long long)c->num_sms * per_sm));
-    k_dns_source<<<grid, 256, 0, st>>>(a);
+    fn<<<grid, 256, 0, st>>>(a);
     RC_CK(cudaGetLastError());
     return RC_OK;
 }
