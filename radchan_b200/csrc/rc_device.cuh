@@ -40,7 +40,7 @@ constexpr int kWarp = 32;
 constexpr int kRefill = 11;  // emitted bundles waiting below which a warp emits the next wave
 constexpr int kRing = kRefill - 1 + kWarp;  // per-warp ring of emitted bundles: those, and a wave
 constexpr int kTileBufs = 3;  // tiles a warp has in flight (tile_bufs)
-constexpr int kGuide = 256;  // buckets of the band-CDF guide tables
+constexpr int kGuide = 1024; // buckets of the band-CDF guide tables
 constexpr int kFeedIdle = 16; // idle lanes that make a warp leave its step loop to take new bundles
 constexpr int kTurnGather = 5; // lanes waiting at scattering events that make a warp draw their turns
 constexpr int kChunkMax = 8;  // tiles a warp claims per work-queue fetch (guided: fewer near the end)
@@ -964,7 +964,7 @@ __device__ __forceinline__ void decode_tile(const DSolve<R> &S, long long item0,
     t.j = d.j - 1;
     t.k = d.k;
     t.v = d.v;
-    t.q = d.h0 / S.rpt;
+    t.q = d.h0 >> (__ffs(S.rpt) - 1);  // rpt: a power of two
 }
 
 // n / d for n < 2^16, d <= 2^15 with m = magic32(d): exact (n d < 2^32).

@@ -917,7 +917,8 @@ struct Impl : ImplBase {
     // few ms per launch (the longest rays), while reordering costs pyramid
     // locality in proportion to the work, hence the limit on tiles.
     static constexpr long long kPrioMaxTiles = 1LL << 22;
-    int enqueue_prio(Slot<R> &s, cudaStream_t st, bool &use) {
+    // desc_dev: the patched descriptor on the device (the slot's, or a batch's).
+    int enqueue_prio(Slot<R> &s, cudaStream_t st, bool &use, const DSolve<R> *desc_dev) {
         std::string *err_ = &c->err;
         use = false;
         const DSolve<R> &d = *s.h_desc;
@@ -952,10 +953,10 @@ struct Impl : ImplBase {
         }
         if (!s.d_nprio) RC_CK(cudaMalloc((void **)&s.d_nprio, 2 * sizeof(unsigned)));
         RC_CK(cudaMemsetAsync(s.d_nprio, 0, 2 * sizeof(unsigned), st));
-        k_prio_kmin<R><<<(nbq + 255) / 256, 256, 0, st>>>(s.d_desc, s.d_kmin);
+        k_prio_kmin<R><<<(nbq + 255) / 256, 256, 0, st>>>(desc_dev, s.d_kmin);
         RC_CK(cudaGetLastError());
         const long long grid = std::max<long long>(1, std::min<long long>((nt + 7) / 8, (long long)c->num_sms * 16));
-        k_prio_tiles<R><<<(unsigned)grid, 256, 0, st>>>(s.d_desc, c->prio_thr, s.d_kmin, s.d_prio, s.d_tprio,
+        k_prio_tiles<R><<<(unsigned)grid, 256, 0, st>>>(desc_dev, c->prio_thr, s.d_kmin, s.d_prio, s.d_tprio,
                                                          s.d_nprio);
         RC_CK(cudaGetLastError());
         memcpy(s.prio_key, key, sizeof(key));
@@ -1141,7 +1142,7 @@ struct Impl : ImplBase {
         // per solve end to end against 28.8-29.1 ms without it
         RC_CK(cudaEventRecord(s.e_march0, s.st));
         bool prio = false;
-        rc = enqueue_prio(s, s.st, prio);
+        rc = enqueue_prio(s, s.st, prio, s.d_desc);
         if (rc) return rc;
         rc = launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, c->block, rpt, s.st, 0,
                           prio ? &s : nullptr, -1, s.h_desc);
@@ -1176,7 +1177,7 @@ struct Impl : ImplBase {
             RC_CK(cudaMemcpyAsync(s.d_tiles, s.h_tiles, 2 * sizeof(long long), cudaMemcpyHostToDevice, s.st));
             RC_CK(cudaEventRecord(s.e_march0, s.st));
             bool prio = false;
-            rc = enqueue_prio(s, s.st, prio);
+            rc = enqueue_prio(s, s.st, prio, s.d_desc);
             if (rc) return rc;
             rc = launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, block, rpt, s.st, minb,
                               prio ? &s : nullptr, -1, s.h_desc);

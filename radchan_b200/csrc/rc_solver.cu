@@ -364,7 +364,7 @@ int rc_debug_fail_next(const char *site, int count) {
 }  // extern "C"
 
 // ---------------------------------------------------------------------------
-// batched solves: many contexts' solves in one persistent launch
+// batched solves: many contexts' solves side by side in one graph
 // ---------------------------------------------------------------------------
 struct rc_batch {
     int device = 0;
@@ -375,6 +375,7 @@ struct rc_batch {
         void *slot;
         int zstart;
         unsigned long long gen;  // the context's generation the captured graph was built with
+        bool prio = false;       // marches with its priority list
     };
     std::vector<Member> m;
     cudaStream_t st = nullptr;
@@ -385,9 +386,7 @@ struct rc_batch {
     cudaGraphExec_t exec = nullptr;
     bool built = false;
     void *d_solves = nullptr, *h_solves = nullptr;
-    long long *d_tiles = nullptr, *h_tiles = nullptr;
     TallyOut *d_outs = nullptr, *h_outs = nullptr;
-    unsigned long long *d_counter = nullptr;
     size_t cap = 0;
     // the members' float results gathered into one buffer and copied to
     // the host once per run (k_copy_segs + one cudaMemcpyAsync)
@@ -412,14 +411,10 @@ int batch_reserve(rc_batch *b, size_t n) {
     if (n <= b->cap) return RC_OK;
     if (b->d_solves) cudaFree(b->d_solves);
     if (b->h_solves) cudaFreeHost(b->h_solves);
-    if (b->d_tiles) cudaFree(b->d_tiles);
-    if (b->h_tiles) cudaFreeHost(b->h_tiles);
     if (b->d_outs) cudaFree(b->d_outs);
     if (b->h_outs) cudaFreeHost(b->h_outs);
     RC_CK(cudaMalloc(&b->d_solves, n * sizeof(DSolve<R>)));
     RC_CK(cudaHostAlloc(&b->h_solves, n * sizeof(DSolve<R>), cudaHostAllocDefault));
-    RC_CK(cudaMalloc((void **)&b->d_tiles, (n + 1) * sizeof(long long)));
-    RC_CK(cudaHostAlloc((void **)&b->h_tiles, (n + 1) * sizeof(long long), cudaHostAllocDefault));
     RC_CK(cudaMalloc((void **)&b->d_outs, n * sizeof(TallyOut)));
     RC_CK(cudaHostAlloc((void **)&b->h_outs, n * sizeof(TallyOut), cudaHostAllocDefault));
     if (b->d_segs) cudaFree(b->d_segs);
@@ -455,44 +450,46 @@ int batch_reserve_members(rc_batch *b) {
     return RC_OK;
 }
 
-// The whole batch on b->st: per member field copy + set-up, one march
-// over every member's tiles, one tally launch, scalars back.
-template <typename R>
-int batch_enqueue(rc_batch *b, bool capturing) {
+// The batch's side streams wait for what b->st has so far / b->st waits for
+// the side streams.
+int batch_fork(rc_batch *b, int ns) {
     std::string *err_ = &b->err;
-    // phase events: inside a captured graph they become event-record nodes
-    auto mark = [&](cudaEvent_t ev) {
-        return capturing ? cudaEventRecordWithFlags(ev, b->st, cudaEventRecordExternal) : cudaEventRecord(ev, b->st);
-    };
+    RC_CK(cudaEventRecord(b->fork, b->st));
+    for (int k = 0; k < ns; ++k) RC_CK(cudaStreamWaitEvent(b->side[k], b->fork, 0));
+    return RC_OK;
+}
+int batch_join(rc_batch *b, int ns) {
+    std::string *err_ = &b->err;
+    for (int k = 0; k < ns; ++k) {
+        RC_CK(cudaEventRecord(b->join[k], b->side[k]));
+        RC_CK(cudaStreamWaitEvent(b->st, b->join[k], 0));
+    }
+    return RC_OK;
+}
+
+// First part of a batch on b->st: per member field copy + set-up.
+template <typename R>
+int batch_enqueue_setup(rc_batch *b) {
+    std::string *err_ = &b->err;
     const size_t n = b->m.size();
     int rc = batch_reserve<R>(b, n);
     if (rc) return rc;
     DSolve<R> *hs = static_cast<DSolve<R> *>(b->h_solves);
-    int rpt_max = 1, block = 256, scat = 0;
-    long long max_cells = 1;
-    b->h_tiles[0] = 0;
-    // host halves: descriptors, tile prefix, tally outputs of every member
+    // host halves: descriptors, tally outputs of every member
     long long maxf = 1;
     for (size_t i = 0; i < n; ++i) {
         rc_ctx *c = b->m[i].ctx;
         Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
-        if (im.nA > 0) scat = 1;  // the scattering variant of the march serves every member
         Slot<R> &s = *static_cast<Slot<R> *>(b->m[i].slot);
         rc = im.prepare_host(s, b->m[i].zstart, c->rpt);
         if (rc) return set_err(err_, rc, c->err);
         hs[i] = *s.h_desc;
         b->h_outs[i] = *s.h_out;
-        b->h_tiles[i + 1] = b->h_tiles[i] + s.h_desc->n_tiles;
-        rpt_max = std::max(rpt_max, c->rpt);
-        if (i == 0) block = c->block;
-        max_cells = std::max(max_cells, im.tally_cells());
         b->h_segs[i] = CopySeg{s.h_T, s.d_T, (long long)im.field_floats()};
         maxf = std::max(maxf, b->h_segs[i].n);
     }
-    // one copy each of the descriptors, tile prefix and tally outputs; every
-    // member's field in one launch that reads the pinned staging directly
+    // one copy each of the descriptors and tally outputs; every member's field in one launch that reads the pinned staging directly
     RC_CK(cudaMemcpyAsync(b->d_solves, hs, n * sizeof(DSolve<R>), cudaMemcpyHostToDevice, b->st));
-    RC_CK(cudaMemcpyAsync(b->d_tiles, b->h_tiles, (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, b->st));
     RC_CK(cudaMemcpyAsync(b->d_outs, b->h_outs, n * sizeof(TallyOut), cudaMemcpyHostToDevice, b->st));
     RC_CK(cudaMemcpyAsync(b->d_segs, b->h_segs, n * sizeof(CopySeg), cudaMemcpyHostToDevice, b->st));
     k_copy_segs<<<dim3((unsigned)std::min<long long>((maxf + 255) / 256, 64), (unsigned)n), 256, 0, b->st>>>(b->d_segs);
@@ -501,8 +498,8 @@ int batch_enqueue(rc_batch *b, bool capturing) {
     // independent chains that run side by side, patching the batch's
     // descriptors in place
     const int ns = (int)std::min<size_t>(n, (size_t)rc_batch::kSideStreams);
-    RC_CK(cudaEventRecord(b->fork, b->st));
-    for (int k = 0; k < ns; ++k) RC_CK(cudaStreamWaitEvent(b->side[k], b->fork, 0));
+    rc = batch_fork(b, ns);
+    if (rc) return rc;
     int rc_members = RC_OK;
     for (size_t i = 0; i < n && !rc_members; ++i) {
         rc_ctx *c = b->m[i].ctx;
@@ -511,16 +508,63 @@ int batch_enqueue(rc_batch *b, bool capturing) {
         rc = im.prepare_device(s, nullptr, true, static_cast<DSolve<R> *>(b->d_solves) + i, b->side[i % ns]);
         if (rc) rc_members = set_err(err_, rc, c->err);
     }
-    for (int k = 0; k < ns; ++k) {
-        RC_CK(cudaEventRecord(b->join[k], b->side[k]));
-        RC_CK(cudaStreamWaitEvent(b->st, b->join[k], 0));
+    rc = batch_join(b, ns);
+    return rc ? rc : rc_members;
+}
+
+// Long-ray priority lists of the members whose list is not up to date, after
+// their set-up on b->st (never captured: a list is kept, see enqueue_prio).
+template <typename R>
+int batch_enqueue_prio(rc_batch *b) {
+    std::string *err_ = &b->err;
+    for (size_t i = 0; i < b->m.size(); ++i) {
+        rc_ctx *c = b->m[i].ctx;
+        Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
+        bool use = false;
+        int rc = im.enqueue_prio(*static_cast<Slot<R> *>(b->m[i].slot), b->st, use,
+                                 static_cast<const DSolve<R> *>(b->d_solves) + i);
+        if (rc) return set_err(err_, rc, c->err);
+        b->m[i].prio = use;
     }
-    if (rc_members) return rc_members;
-    Impl<R> &im0 = *static_cast<Impl<R> *>(b->m[0].ctx->impl);
+    return RC_OK;
+}
+
+// The whole batch on b->st: set-up, every member's march, one tally launch,
+// scalars back.  Each member marches in a launch of its own (the variant
+// whose descriptor is in constant memory, with the member's priority list),
+// round-robin over the side streams: blocks of one march start as those of
+// another run out, so the tails overlap.  One launch over all members read
+// the descriptors through L1 and took no list: 24 small problems 14.2-18 ms,
+// this way BATCHMS.
+template <typename R>
+int batch_enqueue(rc_batch *b, bool capturing) {
+    std::string *err_ = &b->err;
+    // phase events: inside a captured graph they become event-record nodes
+    auto mark = [&](cudaEvent_t ev) {
+        return capturing ? cudaEventRecordWithFlags(ev, b->st, cudaEventRecordExternal) : cudaEventRecord(ev, b->st);
+    };
+    const size_t n = b->m.size();
+    const int ns = (int)std::min<size_t>(n, (size_t)rc_batch::kSideStreams);
+    int rc = batch_enqueue_setup<R>(b);
+    if (!rc && !capturing) rc = batch_enqueue_prio<R>(b);
+    if (rc) return rc;
     RC_CK(mark(b->e_setup));
-    rc = im0.launch_march(static_cast<const DSolve<R> *>(b->d_solves), b->d_tiles, (int)n, b->h_tiles[n],
-                          b->d_counter, block, rpt_max, b->st, 0, nullptr, scat);
-    if (rc) return set_err(err_, rc, b->m[0].ctx->err);
+    rc = batch_fork(b, ns);
+    if (rc) return rc;
+    int rc_members = RC_OK;
+    long long max_cells = 1;
+    for (size_t i = 0; i < n && !rc_members; ++i) {
+        rc_ctx *c = b->m[i].ctx;
+        Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
+        Slot<R> &s = *static_cast<Slot<R> *>(b->m[i].slot);
+        max_cells = std::max(max_cells, im.tally_cells());
+        rc = im.launch_march(static_cast<const DSolve<R> *>(b->d_solves) + i, nullptr, 1, s.h_desc->n_tiles, s.d_counter,
+                             c->block, c->rpt, b->side[i % ns], 0, b->m[i].prio ? &s : nullptr, -1, s.h_desc);
+        if (rc) rc_members = set_err(err_, rc, c->err);
+    }
+    rc = batch_join(b, ns);
+    if (rc || rc_members) return rc ? rc : rc_members;
+    Impl<R> &im0 = *static_cast<Impl<R> *>(b->m[0].ctx->impl);
     RC_CK(mark(b->e_march));
     rc = im0.launch_tally(static_cast<const DSolve<R> *>(b->d_solves), b->d_outs, (int)n, max_cells, b->st);
     if (rc) return set_err(err_, rc, b->m[0].ctx->err);
@@ -605,7 +649,6 @@ int rc_batch_create(int device, int use_graph, rc_batch **out) {
         if ((e = cudaStreamCreateWithFlags(&b->side[k], cudaStreamNonBlocking)) != cudaSuccess) return fail(e);
         if ((e = cudaEventCreateWithFlags(&b->join[k], cudaEventDisableTiming)) != cudaSuccess) return fail(e);
     }
-    if ((e = cudaMalloc((void **)&b->d_counter, sizeof(unsigned long long))) != cudaSuccess) return fail(e);
     (void)err_;
     *out = b;
     return RC_OK;
@@ -679,6 +722,13 @@ int rc_batch_run(rc_batch *b) {
             cudaGraphDestroy(b->graph);
             b->graph = nullptr;
         }
+        // the priority lists need the members' set-up, which runs once more,
+        // outside the graph, when one has to be built
+        rc = b->dbl ? batch_enqueue_setup<double>(b) : batch_enqueue_setup<float>(b);
+        if (!rc) rc = b->dbl ? batch_enqueue_prio<double>(b) : batch_enqueue_prio<float>(b);
+        if (rc) return rc;
+        // the capture rewrites the pinned descriptors that this set-up reads
+        RC_CK(cudaStreamSynchronize(b->st));
         RC_CK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
         rc = b->dbl ? batch_enqueue<double>(b, true) : batch_enqueue<float>(b, true);
         cudaGraph_t g = nullptr;
@@ -759,11 +809,8 @@ int rc_batch_destroy(rc_batch *b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     if (b->d_solves) cudaFree(b->d_solves);
     if (b->h_solves) cudaFreeHost(b->h_solves);
-    if (b->d_tiles) cudaFree(b->d_tiles);
-    if (b->h_tiles) cudaFreeHost(b->h_tiles);
     if (b->d_outs) cudaFree(b->d_outs);
     if (b->h_outs) cudaFreeHost(b->h_outs);
-    if (b->d_counter) cudaFree(b->d_counter);
     if (b->d_segs) cudaFree(b->d_segs);
     if (b->h_segs) cudaFreeHost(b->h_segs);
     if (b->d_pack) cudaFree(b->d_pack);
