@@ -280,8 +280,8 @@ int rc_solve_info_get(rc_ctx *ctx, rc_ticket ticket, rc_solve_info *info);
  * emitted bundles to its lanes in ascending absorption coefficient, so rays
  * traced side by side have similar path lengths (the execution-order part
  * of the reference's srt band sorting, mc_gpu_noint.cu:1270-1294);
- * occupancy: resident 256-thread blocks per SM the register budget must
- * allow (2, 3 or 4).  None of them changes which bundles are traced. */
+ * occupancy: the register budget, as resident 256-thread blocks per SM (2,
+ * 3 or 4; 3 is 72 registers, which also fits seven 128-thread blocks).  None of them changes which bundles are traced. */
 int rc_set_launch(rc_ctx *ctx, int rays_per_thread, int block_threads, int sort_bands, int occupancy);
 int rc_get_launch(rc_ctx *ctx, int *rays_per_thread, int *block_threads, int *sort_bands, int *occupancy);
 /* Long-ray priority of rc_solve_async / rc_solve_device_async.  A bundle
@@ -458,11 +458,11 @@ int rc_slab_comm_destroy(rc_slab_comm *comm);
 /* ---------------- batched solves ---------------- */
 
 typedef struct rc_batch rc_batch;
-/* A batch runs many contexts' solves (uneven grids, tables, photmax) in
- * one persistent work-queue launch; with use_graph the whole sequence
- * (copies + kernels) is captured once and replayed.  The members' fields
- * are copied by one kernel, their set-up kernels run as parallel chains,
- * and the march takes the tiles in natural order.  Every run also gathers
+/* A batch runs many contexts' solves (uneven grids, tables, photmax) side
+ * by side; with use_graph the whole sequence (copies + kernels) is captured
+ * once and replayed.  The members' fields are copied by one kernel, and
+ * their set-up kernels and then their marches run as parallel chains, each
+ * march with its context's launch knobs.  Every run also gathers
  * the members' float results (Q, sigma, wall fluxes) into one buffer
  * copied to the host once, so rc_batch_collect with only Q / sigma copies
  * nothing more. */

@@ -505,7 +505,7 @@ class SlabComm:
 
 
 class Batch:
-    """Many solves of uneven size in one persistent launch (rc_batch_*)."""
+    """Many solves of uneven size side by side in one graph (rc_batch_*)."""
 
     def __init__(self, device=0, use_graph=True):
         self.h = C.c_void_p()

@@ -235,14 +235,6 @@ __device__ __forceinline__ void load_row_if(bool go, const KIRow<double> *p, KIR
         : "l"(p), "r"((int)go));
 }
 
-// A level's words of the descriptor: from the kernel's parameters (constant
-// memory) when the launch marches one solve, else from device memory.
-template <bool ONE>
-__device__ __forceinline__ int4 load_desc(const int4 *p) {
-    if constexpr (ONE) return *p;
-    else return __ldg(p);
-}
-
 // Fraction of a table coordinate: (q mod 256) / 256, exact: the low byte in
 // the mantissa of 2^15 (unit 2^-8), 2^15 subtracted.
 template <typename R>
@@ -540,11 +532,11 @@ __device__ __forceinline__ int crossed_wall(const int3 &c, const int4 &A, const 
 // results.  Returns false when the ray must stop: at a black wall or as a
 // lost ray (the coordinate stays kBlack + wall; retire_ray deposits the rest) or
 // when the budget of the last level is spent.
-template <bool ONE, typename R>
+template <typename R>
 __device__ __forceinline__ bool enter_cell(Ray<R> &r, const DSolve<R> &S) {
     int lev = r.ln >> 20;
-    int4 A = load_desc<ONE>(&S.lva[RC_IX(lev, S.nlev, SITE_LEVEL, S)]);
-    int4 B = load_desc<ONE>(&S.lvb[RC_IX(lev, S.nlev, SITE_LEVEL, S)]);
+    int4 A = S.lva[RC_IX(lev, S.nlev, SITE_LEVEL, S)];
+    int4 B = S.lvb[RC_IX(lev, S.nlev, SITE_LEVEL, S)];
     int3 c = ray_cell(r, A);
     const int code = r.q;
     if (code >= kSpecular) {
@@ -580,8 +572,8 @@ __device__ __forceinline__ bool enter_cell(Ray<R> &r, const DSolve<R> &S) {
         c.z = coarse_index(c.z, L.rz, L.mrz);
         lev += 1;
         r.ln += 1 << 20;
-        A = load_desc<ONE>(&S.lva[lev]);
-        B = load_desc<ONE>(&S.lvb[lev]);
+        A = S.lva[lev];
+        B = S.lvb[lev];
         r.rem = B.y;
     }
     set_cell(r, S, c, A, B);
@@ -592,11 +584,11 @@ __device__ __forceinline__ bool enter_cell(Ray<R> &r, const DSolve<R> &S) {
 // opposite face, with steps left on its level: what enter_cell does for it,
 // without rebuilding what stays.  A channel's rays cross the y and z
 // boundaries in about half of a warp's iterations, one or two lanes at a time.
-template <bool ONE, typename R>
+template <typename R>
 __device__ __forceinline__ void wrap_cell(Ray<R> &r, const DSolve<R> &S) {
     const int lev = RC_IX(r.ln >> 20, S.nlev, SITE_LEVEL, S);
-    const int4 A = load_desc<ONE>(&S.lva[lev]);
-    const int km = load_desc<ONE>(&S.lvb[lev]).x;
+    const int4 A = S.lva[lev];
+    const int km = S.lvb[lev].x;
     const float fjm = (float)A.w, fkm = (float)km;
     if (r.fj < 0.f || r.fj > fjm) {
         const bool hi = r.fj > 0.f;
@@ -640,7 +632,7 @@ __device__ __forceinline__ void absorb(Ray<R> &r, R ds, R absco, R blackpow, boo
 // wall it has reached (:398-399 and its siblings), De -= Ibmax tra ratioI
 // (invTi4 e - 1).  The march retires the stopped rays of a warp together.
 // Returns whether the ray's energy is spent (its transmissivity is then 0).
-template <bool ONE, typename R>
+template <typename R>
 __device__ __forceinline__ bool retire_ray(Ray<R> &r, const DSolve<R> &S) {
     if (r.tra < r.tol) {
         R c2 = (r.Ibmax * r.tra) * r.ratioI;
@@ -655,7 +647,7 @@ __device__ __forceinline__ bool retire_ray(Ray<R> &r, const DSolve<R> &S) {
         e = S.Ibw[RC_IX((size_t)w * S.nB + (r.ln & 0xfffff), 6LL * S.nB, SITE_IBW, S)];
     } else if (t == 4 || t == 6) {  // black wall at a field temperature
         const int lev = RC_IX(r.ln >> 20, S.nlev, SITE_LEVEL, S);
-        const int4 A = load_desc<ONE>(&S.lva[lev]), B = load_desc<ONE>(&S.lvb[lev]);
+        const int4 A = S.lva[lev], B = S.lvb[lev];
         const int im = A.z, jm = A.w, km = B.x;
         const int3 cell = ray_cell(r, A);
         const int idx = w <= RC_EAST    ? (cell.z - 1) * jm + (cell.y - 1)

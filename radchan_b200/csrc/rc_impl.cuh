@@ -171,7 +171,6 @@ struct SlotCommon {
     double *d_q64 = nullptr, *d_var64 = nullptr, *d_qw64 = nullptr, *d_vw64 = nullptr;
     float *d_Qc = nullptr, *d_Sc = nullptr, *d_Wq = nullptr, *d_Ws = nullptr;
     float *h_Qc = nullptr, *h_Sc = nullptr, *h_Wq = nullptr, *h_Ws = nullptr;
-    long long *d_tiles = nullptr, *h_tiles = nullptr;
     unsigned long long *d_counter = nullptr;
     TallyOut *d_out = nullptr, *h_out = nullptr;
     // long-ray priority list (k_prio_tiles): listed tiles, per-tile flag,
@@ -316,8 +315,6 @@ struct Impl : ImplBase {
             hfree(s.h_Sc);
             hfree(s.h_Wq);
             hfree(s.h_Ws);
-            dfree(s.d_tiles);
-            hfree(s.h_tiles);
             dfree(s.d_counter);
             dfree(s.d_out);
             hfree(s.h_out);
@@ -446,8 +443,6 @@ struct Impl : ImplBase {
             RC_CK(cudaHostAlloc((void **)&s.h_Sc, ncf * sizeof(float), cudaHostAllocDefault));
             RC_CK(cudaHostAlloc((void **)&s.h_Wq, nwc * sizeof(float), cudaHostAllocDefault));
             RC_CK(cudaHostAlloc((void **)&s.h_Ws, nwc * sizeof(float), cudaHostAllocDefault));
-            RC_CK(cudaMalloc((void **)&s.d_tiles, 2 * sizeof(long long)));
-            RC_CK(cudaHostAlloc((void **)&s.h_tiles, 2 * sizeof(long long), cudaHostAllocDefault));
             RC_CK(cudaMalloc((void **)&s.d_counter, sizeof(unsigned long long)));
             RC_CK(cudaMalloc((void **)&s.d_out, sizeof(TallyOut)));
             RC_CK(cudaHostAlloc((void **)&s.h_out, sizeof(TallyOut), cudaHostAllocDefault));
@@ -518,9 +513,7 @@ struct Impl : ImplBase {
         c->num_sms = prop.multiProcessorCount;
         smem_opt_in = (int)prop.sharedMemPerBlockOptin;
         for (int v = 0; v < 6; ++v) {
-            RC_CK(cudaFuncSetAttribute(march_fn<false>(2 + v / 2, v & 1), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem_opt_in));
-            RC_CK(cudaFuncSetAttribute(march_fn<true>(2 + v / 2, v & 1), cudaFuncAttributeMaxDynamicSharedMemorySize,
+            RC_CK(cudaFuncSetAttribute(march_fn(2 + v / 2, v & 1), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        smem_opt_in));
         }
         if (p.grey) return set_grey_tables();
@@ -897,11 +890,9 @@ struct Impl : ImplBase {
         return scat ? march_smem_bytes<R, true>(block, rpt_max, nbuf) : march_smem_bytes<R, false>(block, rpt_max, nbuf);
     }
 
-    template <bool ONE>
-    static void (*march_fn(int minb, bool scat))(MarchParams<R, ONE>) {
-        if (scat)
-            return minb <= 2 ? k_march<R, 2, true, ONE> : minb == 3 ? k_march<R, 3, true, ONE> : k_march<R, 4, true, ONE>;
-        return minb <= 2 ? k_march<R, 2, false, ONE> : minb == 3 ? k_march<R, 3, false, ONE> : k_march<R, 4, false, ONE>;
+    static void (*march_fn(int minb, bool scat))(MarchParams<R>) {
+        if (scat) return minb <= 2 ? k_march<R, 2, true> : minb == 3 ? k_march<R, 3, true> : k_march<R, 4, true>;
+        return minb <= 2 ? k_march<R, 2, false> : minb == 3 ? k_march<R, 3, false> : k_march<R, 4, false>;
     }
 
     // Long-ray priority list of a one-solve launch (k_prio_kmin +
@@ -965,48 +956,31 @@ struct Impl : ImplBase {
         return RC_OK;
     }
 
-    // scat: < 0 takes this context's medium (scattering tables set or not);
-    // a launch over several contexts passes whether any of them scatters.
-    // one: the host copy of the descriptor when the launch marches one solve.
-    int launch_march(const DSolve<R> *d_solves, const long long *d_tiles, int nsolves, long long total_tiles,
-                     unsigned long long *d_counter, int block, int rpt_max, cudaStream_t st, int minb = 0,
-                     const Slot<R> *prio = nullptr, int scat = -1, const DSolve<R> *one = nullptr) {
+    // March of n_tiles tiles of the solve with the host descriptor `one` (from
+    // its tile_base on) and the patched descriptor d_desc on the device.
+    int launch_march(const DSolve<R> *d_desc, const DSolve<R> &one, long long n_tiles, unsigned long long *d_counter,
+                     int block, cudaStream_t st, int minb = 0, const Slot<R> *prio = nullptr) {
         std::string *err_ = &c->err;
         RC_FAILPOINT("march");
-        if (minb <= 0) minb = c->minb;
-        const bool sc = scat < 0 ? nA > 0 : scat > 0;
-        MarchArgs a;
-        a.solves = d_solves;
-        a.tile_start = d_tiles;
-        a.nsolves = nsolves;
-        a.total_tiles = total_tiles;
-        a.tile_counter = d_counter;
-        a.rpt_max = rpt_max;
-        a.nbuf = tile_bufs(rpt_max);
-        a.prio_tiles = prio ? prio->d_prio : nullptr;
-        a.tile_prio = prio ? prio->d_tprio : nullptr;
-        a.n_prio = prio ? prio->d_nprio : nullptr;
-        if (one) {
-            MarchParams<R, true> m;
-            m.m = a;
-            m.one = *one;
-            return launch_march_fn(march_fn<true>(minb, sc), m, block, march_smem(block, rpt_max, sc), st);
-        }
-        MarchParams<R, false> m;
-        m.m = a;
-        return launch_march_fn(march_fn<false>(minb, sc), m, block, march_smem(block, rpt_max, sc), st);
-    }
-    template <typename F, typename P>
-    int launch_march_fn(F fn, const P &m, int block, size_t smem, cudaStream_t st) {
-        std::string *err_ = &c->err;
+        auto fn = march_fn(minb > 0 ? minb : c->minb, nA > 0);
+        const size_t smem = march_smem(block, one.rpt, nA > 0);
         if ((int)smem > smem_opt_in) return set_err(err_, RC_E_INVALID, "rays_per_thread too large for shared memory");
         int per_sm = 0;
         RC_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem));
         per_sm = std::max(per_sm, 1);
-        const long long blocks = (m.m.total_tiles + block / kWarp - 1) / (block / kWarp);
+        const long long blocks = (n_tiles + block / kWarp - 1) / (block / kWarp);
         const long long grid = std::max<long long>(1, std::min<long long>((long long)per_sm * c->num_sms, blocks));
-        RC_CK(cudaMemsetAsync(m.m.tile_counter, 0, sizeof(unsigned long long), st));
-        fn<<<(unsigned)grid, block, smem, st>>>(m);
+        RC_CK(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), st));
+        MarchParams<R> p;
+        p.m.desc = d_desc;
+        p.m.total_tiles = n_tiles;
+        p.m.tile_counter = d_counter;
+        p.m.nbuf = tile_bufs(one.rpt);
+        p.m.prio_tiles = prio ? prio->d_prio : nullptr;
+        p.m.tile_prio = prio ? prio->d_tprio : nullptr;
+        p.m.n_prio = prio ? prio->d_nprio : nullptr;
+        p.one = one;
+        fn<<<(unsigned)grid, block, smem, st>>>(p);
         RC_CK(cudaGetLastError());
         return RC_OK;
     }
@@ -1134,9 +1108,6 @@ struct Impl : ImplBase {
         RC_CK(cudaEventRecord(s.e0, s.st));
         rc = prepare(s, device_ptr ? T : nullptr, zstart, rpt, s.st);
         if (rc) return rc;
-        s.h_tiles[0] = 0;
-        s.h_tiles[1] = s.h_desc->n_tiles;
-        RC_CK(cudaMemcpyAsync(s.d_tiles, s.h_tiles, 2 * sizeof(long long), cudaMemcpyHostToDevice, s.st));
         // the long-ray priority list (built once per slot, then reused):
         // also while the other slot's solve runs, where it measured 28.1 ms
         // per solve end to end against 28.8-29.1 ms without it
@@ -1144,8 +1115,7 @@ struct Impl : ImplBase {
         bool prio = false;
         rc = enqueue_prio(s, s.st, prio, s.d_desc);
         if (rc) return rc;
-        rc = launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, c->block, rpt, s.st, 0,
-                          prio ? &s : nullptr, -1, s.h_desc);
+        rc = launch_march(s.d_desc, *s.h_desc, s.h_desc->n_tiles, s.d_counter, c->block, s.st, 0, prio ? &s : nullptr);
         if (rc) return rc;
         RC_CK(cudaEventRecord(s.e_march1, s.st));
         rc = launch_tally(s.d_desc, s.d_out, 1, tally_cells(), s.st);
@@ -1172,15 +1142,12 @@ struct Impl : ImplBase {
         for (int rep = 0; rep < 3; ++rep) {
             int rc = prepare(s, nullptr, zstart, rpt, s.st);
             if (rc) return rc;
-            s.h_tiles[0] = 0;
-            s.h_tiles[1] = s.h_desc->n_tiles;
-            RC_CK(cudaMemcpyAsync(s.d_tiles, s.h_tiles, 2 * sizeof(long long), cudaMemcpyHostToDevice, s.st));
             RC_CK(cudaEventRecord(s.e_march0, s.st));
             bool prio = false;
             rc = enqueue_prio(s, s.st, prio, s.d_desc);
             if (rc) return rc;
-            rc = launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, block, rpt, s.st, minb,
-                              prio ? &s : nullptr, -1, s.h_desc);
+            rc = launch_march(s.d_desc, *s.h_desc, s.h_desc->n_tiles, s.d_counter, block, s.st, minb,
+                              prio ? &s : nullptr);
             if (rc) return rc;
             RC_CK(cudaEventRecord(s.e_march1, s.st));
             RC_CK(cudaEventSynchronize(s.e_march1));

@@ -372,8 +372,8 @@ __global__ void k_trace(const DSolve<R> *Sp, int n, const rc_bundle_id *ids, rc_
         bool active = true;
         while (active) {
             if (r.q >= kSpecular || r.rem <= 0) {
-                if (r.q == kPeriodic && r.rem > 0) wrap_cell<false>(r, S);
-                else active = enter_cell<false>(r, S);
+                if (r.q == kPeriodic && r.rem > 0) wrap_cell(r, S);
+                else active = enter_cell(r, S);
             }
             if (!active || r.q >= kSpecular) continue;
             if (ns < max_cells && cells) {
@@ -388,7 +388,7 @@ __global__ void k_trace(const DSolve<R> *Sp, int n, const rc_bundle_id *ids, rc_
             if (SCAT && active && qs.dist < (R)0) scatter_turn(r, ctr, ks, qs, S);
             ns++;
         }
-        const bool spent = retire_ray<false>(r, S);
+        const bool spent = retire_ray(r, S);
         rec.nsteps = ns;
         rec.end_level = r.ln >> 20;
         rec.tra = spent ? 0.f : (float)r.tra;

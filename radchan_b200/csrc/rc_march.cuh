@@ -20,7 +20,7 @@ namespace rc {
 //     kFeedIdle lanes are idle, then retires the rays that stopped and hands
 //     those lanes the next emitted bundles (warp ballot + prefix count);
 //   * two to four tiles can be in flight (tile_bufs): once every bundle of a tile has been
-//     emitted, the warp fetches the next tile (of the same solve) and keeps
+//     emitted, the warp fetches the next tile and keeps
 //     emitting from it while the last rays of earlier tiles finish, so long
 //     rays do not leave the other lanes idle;
 //   * each bundle's FP64 tally goes to its own shared-memory slot; when a
@@ -36,14 +36,11 @@ namespace rc {
 // keeps these entries and adds a small side array (see WarpShared).
 
 struct MarchArgs {
-    const void *solves;          // DSolve<R>[nsolves] (run-time fields patched on the device)
-    const long long *tile_start; // [nsolves+1] exclusive prefix of tiles
-    int nsolves;
+    const void *desc;            // DSolve<R> on the device (run-time fields patched)
     long long total_tiles;
     unsigned long long *tile_counter;
-    int rpt_max;
     int nbuf;  // tiles a warp has in flight (tile_bufs)
-    // long-ray priority (one solve only; NULL: tiles in natural order): the
+    // long-ray priority (NULL: tiles in natural order): the
     // first n_prio[0] claims take the head of prio_tiles[], the next
     // n_prio[1] its end (backwards), the rest take the natural order and skip
     // the tiles whose tile_prio byte is set
@@ -51,16 +48,14 @@ struct MarchArgs {
     const unsigned char *tile_prio;
     const unsigned *n_prio;
 };
-// A launch over one solve carries its descriptor in the kernel's parameters:
-// what the march reads of it then comes from constant memory (operands and
-// uniform registers) instead of loads through L1 into registers.  The run-time
-// values (Ibmax, table row) are still read from the copy in device memory.
-template <typename R, bool ONE>
-struct MarchParams {
-    MarchArgs m;
-};
+// A launch carries its solve's descriptor in the kernel's parameters: what the
+// march reads of it comes from constant memory (operands and uniform
+// registers) instead of loads through L1 into registers.  The run-time values
+// (Ibmax, table row) are read from the copy in device memory.  (A launch over
+// several solves, with the descriptors in device memory, ran 30% slower per
+// step: several solves are several launches, side by side.)
 template <typename R>
-struct MarchParams<R, true> {
+struct MarchParams {
     MarchArgs m;
     DSolve<R> one;
 };
@@ -161,17 +156,6 @@ struct WarpShared<R, true> {
     uint32_t nev[kWarp];
 };
 
-// Index of the solve owning a global tile (tile_start is an exclusive prefix).
-__device__ __forceinline__ int solve_of_tile(const long long *tile_start, int nsolves, unsigned long long tile) {
-    int lo = 0, hi = nsolves;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((unsigned long long)tile_start[mid] <= tile) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
 __device__ __forceinline__ void flush_counters(DScalars *sc, unsigned long long &nsteps, unsigned long long &nbund,
                                                int lane) {
     unsigned long long st = nsteps, nb = nbund;
@@ -186,12 +170,6 @@ __device__ __forceinline__ void flush_counters(DScalars *sc, unsigned long long 
     nsteps = nbund = 0;
 }
 
-template <bool ONE, typename R>
-__device__ __forceinline__ const DSolve<R> &one_or(const MarchParams<R, ONE> &prm, const DSolve<R> &D) {
-    if constexpr (ONE) return prm.one;
-    else return D;
-}
-
 // Ring position of a running index (below 2 kRing).
 __device__ __forceinline__ int ring_at(int i) { return i < kRing ? i : i - kRing; }
 
@@ -202,8 +180,8 @@ __device__ __forceinline__ int ring_at(int i) { return i < kRing ? i : i - kRing
 // blocks onto an SM, 72 seven 128-thread blocks, 128 two 256-thread blocks.
 constexpr int march_regs(int minb) { return minb >= 4 ? 64 : minb == 3 ? 72 : 128; }
 
-template <typename R, int MINB, bool SCAT, bool ONE>
-__global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(const __grid_constant__ MarchParams<R, ONE> prm) {
+template <typename R, int MINB, bool SCAT>
+__global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(const __grid_constant__ MarchParams<R> prm) {
     const MarchArgs &a = prm.m;
     extern __shared__ __align__(16) unsigned char smem[];
     // volatile: kept in a register instead of read again at every use
@@ -213,19 +191,16 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
     const int nwarps = blockDim.x >> 5;
     WarpShared<R, SCAT> *ws = reinterpret_cast<WarpShared<R, SCAT> *>(smem) + warp;
     const size_t wbytes = ((sizeof(WarpShared<R, SCAT>) * nwarps) + 15) & ~(size_t)15;
-    const int pool_max = kWarp * a.rpt_max;
-    double *slots0 = reinterpret_cast<double *>(smem + wbytes) + (size_t)warp * a.nbuf * pool_max;
-    const DSolve<R> *solves = reinterpret_cast<const DSolve<R> *>(a.solves);
+    const DSolve<R> &S = prm.one;
+    double *slots0 = reinterpret_cast<double *>(smem + wbytes) + (size_t)warp * a.nbuf * (kWarp * S.rpt);
+    const DSolve<R> &D = *reinterpret_cast<const DSolve<R> *>(a.desc);  // with the run-time values
     const unsigned lt = (1u << lane) - 1u;
-    const DSolve<R> *Sp = solves;
 
     // warp-uniform state
-    int cur_solve = -1;
     unsigned busy = 0u;     // bit p: buffer p holds a tile not yet reduced
     int epar = -1;          // buffer being emitted from (-1: every bundle of the busy buffers is emitted)
     int next_b = 0, head = 0, count = 0;
     bool drained = false;   // no more tiles
-    unsigned long long pending = ~0ull;  // fetched tile waiting for a solve switch
     // tiles claimed from the queue but not started: chunk_left from chunk_next on
     unsigned long long chunk_next = 0;
     int chunk_left = 0;
@@ -250,76 +225,58 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
                 const volatile unsigned *np = a.n_prio;
                 const unsigned nsolo = np ? np[0] : 0u, nprio = np ? nsolo + np[1] : 0u;
                 const unsigned long long total = (unsigned long long)a.total_tiles + nprio;
-                unsigned long long tile = ONE ? ~0ull : pending;
-                if (tile == ~0ull) {
-                    // ends: every pass advances chunk_next or the shared
-                    // counter, and a claim at or past `total` ends the queue
-                    for (;;) {
-                        if (chunk_left <= 0) {
-                            // guided self-scheduling: claim up to kChunkMax
-                            // consecutive tiles (usually of one solve), so a
-                            // warp keeps its tiles of the same solve in
-                            // flight; claim fewer as the queue drains to keep
-                            // the tail short, and the longest rays one by one
-                            if (lane == 0) {
-                                const unsigned long long seen = *(volatile unsigned long long *)a.tile_counter;
-                                const unsigned long long rem = seen < total ? total - seen : 0ull;
-                                const unsigned long long k = rem / (4ull * gridDim.x * nwarps);
-                                chunk_left = seen < nsolo ? 1 : (int)max(1ull, min((unsigned long long)kChunkMax, k));
-                                chunk_next = atomicAdd(a.tile_counter, (unsigned long long)chunk_left);
-                            }
-                            chunk_next = __shfl_sync(0xffffffffu, chunk_next, 0);
-                            chunk_left = __shfl_sync(0xffffffffu, chunk_left, 0);
+                unsigned long long tile;
+                // ends: every pass advances chunk_next or the shared
+                // counter, and a claim at or past `total` ends the queue
+                for (;;) {
+                    if (chunk_left <= 0) {
+                        // guided self-scheduling: claim up to kChunkMax
+                        // consecutive tiles (neighbouring cells); claim
+                        // fewer as the queue drains to keep the tail short,
+                        // and the longest rays one by one
+                        if (lane == 0) {
+                            const unsigned long long seen = *(volatile unsigned long long *)a.tile_counter;
+                            const unsigned long long rem = seen < total ? total - seen : 0ull;
+                            const unsigned long long k = rem / (4ull * gridDim.x * nwarps);
+                            chunk_left = seen < nsolo ? 1 : (int)max(1ull, min((unsigned long long)kChunkMax, k));
+                            chunk_next = atomicAdd(a.tile_counter, (unsigned long long)chunk_left);
                         }
-                        tile = chunk_next++;
-                        chunk_left--;
-                        if (tile >= total) {
-                            tile = total;
-                            break;
-                        }
-                        if (!np) break;
-                        if (tile < nprio) {
-                            hold = tile < nsolo;
-                            tile = __ldg(a.prio_tiles + (hold ? tile : (unsigned long long)a.total_tiles - 1 - (tile - nsolo)));
-                            break;
-                        }
-                        if (!__ldg(a.tile_prio + (tile - nprio))) {
-                            tile -= nprio;
-                            break;
-                        }
-                        // a listed tile met again in natural order: claim the next
+                        chunk_next = __shfl_sync(0xffffffffu, chunk_next, 0);
+                        chunk_left = __shfl_sync(0xffffffffu, chunk_left, 0);
                     }
+                    tile = chunk_next++;
+                    chunk_left--;
+                    if (tile >= total) {
+                        tile = total;
+                        break;
+                    }
+                    if (!np) break;
+                    if (tile < nprio) {
+                        hold = tile < nsolo;
+                        tile = __ldg(a.prio_tiles + (hold ? tile : (unsigned long long)a.total_tiles - 1 - (tile - nsolo)));
+                        break;
+                    }
+                    if (!__ldg(a.tile_prio + (tile - nprio))) {
+                        tile -= nprio;
+                        break;
+                    }
+                    // a listed tile met again in natural order: claim the next
                 }
                 if (tile >= (unsigned long long)a.total_tiles) {
                     drained = true;
-                    pending = ~0ull;
                 } else {
-                    const int so = ONE ? 0 : solve_of_tile(a.tile_start, a.nsolves, tile);
-                    if (so != cur_solve && busy) {
-                        pending = tile;  // switch solves only once every buffer is reduced
-                    } else {
-                        pending = ~0ull;
-                        if (so != cur_solve) {
-                            if (cur_solve >= 0) flush_counters(Sp->sc, nsteps, nbund, lane);
-                            Sp = solves + so;
-                            cur_solve = so;
-                        }
-                        const long long t0 = (long long)(ONE ? tile : tile - (unsigned long long)a.tile_start[so]);
-                        if (lane == 0) decode_tile(one_or<ONE>(prm, *Sp), (t0 + Sp->tile_base) * kWarp, ws->tile[fpar]);
-                        double *sl = slots0 + fpar * pool_max;
-                        for (int b = lane; b < kWarp * Sp->rpt; b += kWarp) sl[b] = 0.0;
-                        busy |= 1u << fpar;
-                        epar = fpar;
-                        next_b = 0;
-                        __syncwarp();
-                    }
+                    if (lane == 0) decode_tile(S, ((long long)tile + S.tile_base) * kWarp, ws->tile[fpar]);
+                    double *sl = slots0 + fpar * (kWarp * S.rpt);
+                    for (int b = lane; b < kWarp * S.rpt; b += kWarp) sl[b] = 0.0;
+                    busy |= 1u << fpar;
+                    epar = fpar;
+                    next_b = 0;
+                    __syncwarp();
                 }
             }
         }
-        const DSolve<R> &D = *Sp;  // with the run-time values
-        const DSolve<R> &S = one_or<ONE>(prm, D);
         const int rpt = S.rpt;
-        const int lrpt = __ffs(rpt) - 1;  // rpt is a power of two
+        const int lrpt = __ffs(rpt) - 1;
         const int pool = kWarp * rpt;
         // ---- converged emission wave: one bundle per lane
         if (count < kRefill && epar >= 0) {
@@ -432,8 +389,8 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
                 bool go = active;
                 if constexpr (SCAT) go = active && !(qs.dist < (R)0);
                 if (go && (r.q >= kSpecular || r.rem <= 0)) {
-                    if (r.q == kPeriodic && r.rem > 0) wrap_cell<ONE>(r, S);
-                    else active = enter_cell<ONE>(r, S);
+                    if (r.q == kPeriodic && r.rem > 0) wrap_cell(r, S);
+                    else active = enter_cell(r, S);
                 }
                 go = go && active && r.q < kSpecular;
                 const bool above = march_step<R, SCAT>(r, qs, S, go);
@@ -459,9 +416,9 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
             bool last = false;
             if (am != amask) {
                 if (((amask & ~am) >> lane) & 1u) {
-                    retire_ray<ONE>(r, S);
+                    retire_ray(r, S);
                     nsteps += S.steps_to[r.ln >> 20] - r.rem;
-                    slots0[(myslot >> 12) * pool_max + (myslot & 0xfff)] = r.De;
+                    slots0[(myslot >> 12) * pool + (myslot & 0xfff)] = r.De;
                     last = atomicSub(&ws->tile[myslot >> 12].out, 1) == 1;
                 }
                 amask = am;
@@ -496,7 +453,7 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
             while (ready) {
                 const int par = __ffs(ready) - 1;
                 ready &= ready - 1u;
-                const double *sl = slots0 + par * pool_max;
+                const double *sl = slots0 + par * pool;
                 double s = 0.0;
                 for (int h = 0; h < rpt; ++h) s += sl[lane * rpt + h];
                 const int base = lane >> lgs << lgs;
@@ -511,17 +468,17 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
         }
         if (drained && !busy) break;
     }
-    if (cur_solve >= 0) flush_counters(Sp->sc, nsteps, nbund, lane);
+    flush_counters(S.sc, nsteps, nbund, lane);
 }
 
 // Tiles a warp keeps in flight.  A tile's slots are held until its longest
 // ray has finished, and with every buffer held the warp runs out of bundles.
-constexpr int tile_bufs(int rpt_max) { return rpt_max <= 4 ? kTileBufs : 2; }
+constexpr int tile_bufs(int rpt) { return rpt <= 4 ? kTileBufs : 2; }
 
 template <typename R, bool SCAT>
-constexpr size_t march_smem_bytes(int block, int rpt_max, int nbuf) {
+constexpr size_t march_smem_bytes(int block, int rpt, int nbuf) {
     return ((((size_t)sizeof(WarpShared<R, SCAT>) * (block / kWarp)) + 15) & ~(size_t)15) +
-           (size_t)(block / kWarp) * nbuf * kWarp * rpt_max * sizeof(double);
+           (size_t)(block / kWarp) * nbuf * kWarp * rpt * sizeof(double);
 }
 
 }  // namespace rc

@@ -10,12 +10,15 @@
 //     budget; every admitted request takes a pooled solver context whose
 //     grid, tables and buffers stay resident between requests of the same
 //     problem class (everything but photmax and the seed equal);
-//   * one scheduler thread drives the GPU in quanta: a quantum is one
-//     persistent march launch whose work queue holds tiles of every running
-//     request -- by default the requests with the least remaining work
-//     first, above a floor share for everyone (or equal shares, processor
-//     sharing) -- so a request that arrives while long solves run joins the
-//     next quantum instead of queueing behind them;
+//   * one scheduler thread drives the GPU in quanta: a quantum marches tiles
+//     of every running request, one launch per request side by side on the
+//     quantum's march streams -- by default the requests with the least
+//     remaining work first, above a floor share for everyone (or equal
+//     shares, processor sharing) -- so a request that arrives while long
+//     solves run joins the next quantum instead of queueing behind them.
+//     (One launch over all requests read the descriptors through L1 and
+//     drained its warps at every change of request: 16 small requests took
+//     12.3-13.0 ms, this way 9.2-9.8 ms);
 //   * quanta go round-robin to eight streams, so a quantum's tail (its
 //     longest rays: in near-transparent bands a ray can take up to the last
 //     level's step budget, maxs, tens of milliseconds) overlaps the next
@@ -127,12 +130,12 @@ struct rc_server {
     static constexpr int kNQ = 8;
     cudaStream_t qst[kNQ] = {};
     int cap = 0;
-    DSolve<float> *d_solves[kNQ] = {};
-    long long *d_tiles[kNQ] = {};
-    long long *d_base[kNQ] = {};
-    long long *h_tiles[kNQ] = {};
-    long long *h_base[kNQ] = {};
-    unsigned long long *d_counter[kNQ] = {};
+    unsigned long long *d_counter[kNQ] = {};  // one tile counter per march of the quantum
+    // the marches of a quantum, one launch per request, run side by side on
+    // these streams, forked from and joined back into the quantum's stream
+    static constexpr int kMS = 4;
+    cudaStream_t ms[kNQ][kMS] = {};
+    cudaEvent_t ms_done[kNQ][kMS] = {};
     cudaEvent_t pre_done[kNQ] = {};  // prelude (set-up, descriptors) of the parity's latest quantum done
     cudaEvent_t mend[kNQ] = {};      // march of the parity's latest quantum done
     bool q_used[kNQ] = {};
@@ -147,11 +150,6 @@ struct rc_server {
 };
 
 namespace rc_detail {
-
-__global__ void k_set_tile_base(DSolve<float> *d, const long long *base, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) d[i].tile_base = base[i];
-}
 
 // Problem class: everything that fixes a context's device layout.
 std::string class_key(const rc_params &p, int table_set) {
@@ -217,23 +215,13 @@ int grow_quantum_buffers(rc_server *sv, int n) {
     if (n <= sv->cap) return RC_OK;
     for (int i = 0; i < rc_server::kNQ; ++i) RC_CK(cudaStreamSynchronize(sv->qst[i]));
     for (int i = 0; i < rc_server::kNQ; ++i) {
-        if (sv->d_solves[i]) cudaFree(sv->d_solves[i]);
-        if (sv->d_tiles[i]) cudaFree(sv->d_tiles[i]);
-        if (sv->d_base[i]) cudaFree(sv->d_base[i]);
-        if (sv->h_tiles[i]) cudaFreeHost(sv->h_tiles[i]);
-        if (sv->h_base[i]) cudaFreeHost(sv->h_base[i]);
-        sv->d_solves[i] = nullptr;
-        sv->d_tiles[i] = sv->d_base[i] = sv->h_tiles[i] = sv->h_base[i] = nullptr;
+        if (sv->d_counter[i]) cudaFree(sv->d_counter[i]);
+        sv->d_counter[i] = nullptr;
     }
     sv->cap = 0;
     const int c = std::max(n, 64);
-    for (int i = 0; i < rc_server::kNQ; ++i) {
-        RC_CK(cudaMalloc((void **)&sv->d_solves[i], c * sizeof(DSolve<float>)));
-        RC_CK(cudaMalloc((void **)&sv->d_tiles[i], (c + 1) * sizeof(long long)));
-        RC_CK(cudaMalloc((void **)&sv->d_base[i], c * sizeof(long long)));
-        RC_CK(cudaHostAlloc((void **)&sv->h_tiles[i], (c + 1) * sizeof(long long), cudaHostAllocDefault));
-        RC_CK(cudaHostAlloc((void **)&sv->h_base[i], c * sizeof(long long), cudaHostAllocDefault));
-    }
+    for (int i = 0; i < rc_server::kNQ; ++i)
+        RC_CK(cudaMalloc((void **)&sv->d_counter[i], c * sizeof(unsigned long long)));
     sv->cap = c;
     return RC_OK;
 }
@@ -372,17 +360,16 @@ int start_stage(rc_server *sv, SrvReq *r, cudaStream_t st) {
     return RC_OK;
 }
 
-// Prelude and march of one quantum on stream qst[par]: equal shares of every
-// marching request's remaining tiles in one persistent launch.  Set-up work
-// of new stages was enqueued on the same stream just before.
+// Prelude of one quantum on stream qst[par] and its marches, joined back into
+// that stream: a share of every marching request's remaining tiles, in one
+// launch each.  Set-up work of new stages was enqueued on the same stream just
+// before.
 int run_quantum(rc_server *sv, const std::vector<SrvReq *> &marching, int par) {
     Range nv("rc_server quantum");
     std::string *err_ = &sv->err;
     RC_FAILPOINT("quantum");
     const int n = (int)marching.size();
     cudaStream_t st = sv->qst[par];
-    long long *ht = sv->h_tiles[par], *hb = sv->h_base[par];
-    ht[0] = 0;
     long long qt;
     int policy;
     {
@@ -421,30 +408,29 @@ int run_quantum(rc_server *sv, const std::vector<SrvReq *> &marching, int par) {
             budget -= more;
         }
     }
-    int rpt_max = 1;
-    for (int i = 0; i < n; ++i) {
-        SrvReq *r = marching[i];
-        hb[i] = r->next_tile;
-        ht[i + 1] = ht[i] + take[i];
-        r->next_tile += take[i];
-        rpt_max = std::max(rpt_max, r->ctx->rpt);
-        RC_CK(cudaMemcpyAsync(sv->d_solves[par] + i, r->slot->d_desc, sizeof(DSolve<float>),
-                              cudaMemcpyDeviceToDevice, st));
-    }
-    RC_CK(cudaMemcpyAsync(sv->d_tiles[par], ht, (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, st));
-    RC_CK(cudaMemcpyAsync(sv->d_base[par], hb, n * sizeof(long long), cudaMemcpyHostToDevice, st));
-    k_set_tile_base<<<(n + 127) / 128, 128, 0, st>>>(sv->d_solves[par], sv->d_base[par], n);
-    RC_CK(cudaGetLastError());
     RC_CK(cudaEventRecord(sv->pre_done[par], st));
-    if (ht[n] > 0) {
-        Impl<float> &im0 = *static_cast<Impl<float> *>(marching[0]->ctx->impl);
-        int scat = 0;  // the scattering variant of the march when any request's medium scatters
-        for (int i = 0; i < n; ++i)
-            if (static_cast<Impl<float> *>(marching[i]->ctx->impl)->nA > 0) scat = 1;
-        const int rc = im0.launch_march(sv->d_solves[par], sv->d_tiles[par], n, ht[n], sv->d_counter[par],
-                                        marching[0]->ctx->block, rpt_max, st, 0, nullptr, scat);
-        if (rc) return set_err(err_, rc, marching[0]->ctx->err);
+    // one launch per request over its share of tiles
+    const int nms = std::min(n, rc_server::kMS);
+    for (int k = 0; k < nms; ++k) RC_CK(cudaStreamWaitEvent(sv->ms[par][k], sv->pre_done[par], 0));
+    int rc_march = RC_OK;
+    for (int i = 0; i < n && !rc_march; ++i) {
+        SrvReq *r = marching[i];
+        if (take[i] <= 0) continue;
+        Impl<float> &im = *static_cast<Impl<float> *>(r->ctx->impl);
+        DSolve<float> d = *r->slot->h_desc;
+        d.tile_base = r->next_tile;
+        r->next_tile += take[i];
+        rc_march = im.launch_march(r->slot->d_desc, d, take[i], sv->d_counter[par] + i, r->ctx->block,
+                                   sv->ms[par][i % nms]);
+        if (rc_march) set_err(err_, rc_march, r->ctx->err);
     }
+    for (int k = 0; k < nms; ++k) {
+        // a join that cannot be recorded is replaced by waiting on the host
+        if (cudaEventRecord(sv->ms_done[par][k], sv->ms[par][k]) != cudaSuccess ||
+            cudaStreamWaitEvent(st, sv->ms_done[par][k], 0) != cudaSuccess)
+            cudaStreamSynchronize(sv->ms[par][k]);
+    }
+    if (rc_march) return rc_march;
     RC_CK(cudaEventRecord(sv->mend[par], st));
     return RC_OK;
 }
@@ -726,13 +712,16 @@ int rc_server_create(int device, double hbm_budget_bytes, int max_inflight, rc_s
     bool ok = cudaStreamCreateWithFlags(&sv->st, cudaStreamNonBlocking) == cudaSuccess;
     for (int i = 0; i < rc_server::kNQ && ok; ++i)
         ok = cudaStreamCreateWithFlags(&sv->qst[i], cudaStreamNonBlocking) == cudaSuccess &&
-             cudaMalloc((void **)&sv->d_counter[i], sizeof(unsigned long long)) == cudaSuccess &&
              cudaEventCreateWithFlags(&sv->pre_done[i], cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&sv->mend[i], cudaEventDisableTiming) == cudaSuccess;
     ok = ok && cudaEventCreateWithFlags(&sv->fork, cudaEventDisableTiming) == cudaSuccess;
     for (int i = 0; i < rc_server::kSide && ok; ++i)
         ok = cudaStreamCreateWithFlags(&sv->side[i], cudaStreamNonBlocking) == cudaSuccess &&
              cudaEventCreateWithFlags(&sv->join[i], cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; i < rc_server::kNQ * rc_server::kMS && ok; ++i)
+        ok = cudaStreamCreateWithFlags(&sv->ms[i / rc_server::kMS][i % rc_server::kMS], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&sv->ms_done[i / rc_server::kMS][i % rc_server::kMS], cudaEventDisableTiming) ==
+                 cudaSuccess;
     if (!ok) {
         rc_server_destroy(sv);
         return set_err(nullptr, RC_E_CUDA, "server stream/event creation failed");
@@ -917,11 +906,13 @@ int rc_server_destroy(rc_server *sv) {
     for (auto &kv : sv->reqs)
         if (kv.second->ev) cudaEventDestroy(kv.second->ev);
     for (int i = 0; i < rc_server::kNQ; ++i) {
-        if (sv->d_solves[i]) cudaFree(sv->d_solves[i]);
-        if (sv->d_tiles[i]) cudaFree(sv->d_tiles[i]);
-        if (sv->d_base[i]) cudaFree(sv->d_base[i]);
-        if (sv->h_tiles[i]) cudaFreeHost(sv->h_tiles[i]);
-        if (sv->h_base[i]) cudaFreeHost(sv->h_base[i]);
+        for (int k = 0; k < rc_server::kMS; ++k) {
+            if (sv->ms[i][k]) {
+                cudaStreamSynchronize(sv->ms[i][k]);
+                cudaStreamDestroy(sv->ms[i][k]);
+            }
+            if (sv->ms_done[i][k]) cudaEventDestroy(sv->ms_done[i][k]);
+        }
         if (sv->d_counter[i]) cudaFree(sv->d_counter[i]);
         if (sv->pre_done[i]) cudaEventDestroy(sv->pre_done[i]);
         if (sv->mend[i]) cudaEventDestroy(sv->mend[i]);

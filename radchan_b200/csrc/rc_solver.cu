@@ -1,5 +1,5 @@
-// rc_solver.cu -- C ABI of solver contexts, batched solves in one
-// persistent launch (optionally a CUDA graph), bundle traces, the launch
+// rc_solver.cu -- C ABI of solver contexts, batched solves side by side
+// (optionally as one CUDA graph), bundle traces, the launch
 // autotuner and the allocation-free solve, behind radchan.h.  The context
 // implementation is in rc_impl.cuh.
 #include "rc_impl.cuh"
@@ -488,7 +488,8 @@ int batch_enqueue_setup(rc_batch *b) {
         b->h_segs[i] = CopySeg{s.h_T, s.d_T, (long long)im.field_floats()};
         maxf = std::max(maxf, b->h_segs[i].n);
     }
-    // one copy each of the descriptors and tally outputs; every member's field in one launch that reads the pinned staging directly
+    // one copy each of the descriptors and tally outputs; every member's
+    // field in one launch that reads the pinned staging directly
     RC_CK(cudaMemcpyAsync(b->d_solves, hs, n * sizeof(DSolve<R>), cudaMemcpyHostToDevice, b->st));
     RC_CK(cudaMemcpyAsync(b->d_outs, b->h_outs, n * sizeof(TallyOut), cudaMemcpyHostToDevice, b->st));
     RC_CK(cudaMemcpyAsync(b->d_segs, b->h_segs, n * sizeof(CopySeg), cudaMemcpyHostToDevice, b->st));
@@ -535,7 +536,7 @@ int batch_enqueue_prio(rc_batch *b) {
 // round-robin over the side streams: blocks of one march start as those of
 // another run out, so the tails overlap.  One launch over all members read
 // the descriptors through L1 and took no list: 24 small problems 14.2-18 ms,
-// this way BATCHMS.
+// this way 10.5 ms (march).
 template <typename R>
 int batch_enqueue(rc_batch *b, bool capturing) {
     std::string *err_ = &b->err;
@@ -558,8 +559,8 @@ int batch_enqueue(rc_batch *b, bool capturing) {
         Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
         Slot<R> &s = *static_cast<Slot<R> *>(b->m[i].slot);
         max_cells = std::max(max_cells, im.tally_cells());
-        rc = im.launch_march(static_cast<const DSolve<R> *>(b->d_solves) + i, nullptr, 1, s.h_desc->n_tiles, s.d_counter,
-                             c->block, c->rpt, b->side[i % ns], 0, b->m[i].prio ? &s : nullptr, -1, s.h_desc);
+        rc = im.launch_march(static_cast<const DSolve<R> *>(b->d_solves) + i, *s.h_desc, s.h_desc->n_tiles, s.d_counter,
+                             c->block, b->side[i % ns], 0, b->m[i].prio ? &s : nullptr);
         if (rc) rc_members = set_err(err_, rc, c->err);
     }
     rc = batch_join(b, ns);
@@ -912,16 +913,13 @@ int solve_noalloc_t(rc_ctx *c, const float *T_dev, int zstart, double *q64, doub
     o->Wq = s.d_Wq;
     o->Ws = s.d_Ws;
     RC_CK(cudaMemcpyAsync(s.d_out, s.h_out, sizeof(TallyOut), cudaMemcpyHostToDevice, st));
-    s.h_tiles[0] = 0;
-    s.h_tiles[1] = s.h_desc->n_tiles;
-    RC_CK(cudaMemcpyAsync(s.d_tiles, s.h_tiles, 2 * sizeof(long long), cudaMemcpyHostToDevice, st));
     // The tally writes only the walls whose flux is computed; the others read
     // 0, as the allocating entry points return them.
     const int nwalls = s.h_desc->nwalls;
     const size_t wall_bytes = 2 * (size_t)s.h_desc->nwc * sizeof(double);
     if (nwalls < 2 && qw64) RC_CK(cudaMemsetAsync(qw64, 0, wall_bytes, st));
     if (nwalls < 2 && vw64) RC_CK(cudaMemsetAsync(vw64, 0, wall_bytes, st));
-    rc = im.launch_march(s.d_desc, s.d_tiles, 1, s.h_desc->n_tiles, s.d_counter, c->block, rpt, st, 0, nullptr, -1, s.h_desc);
+    rc = im.launch_march(s.d_desc, *s.h_desc, s.h_desc->n_tiles, s.d_counter, c->block, st);
     if (rc) return rc;
     rc = im.launch_tally(s.d_desc, s.d_out, 1, im.tally_cells(), st);
     if (rc) return rc;
