@@ -6,8 +6,8 @@
 // memory_copy_noint.cu): the grid, the tables and the Planck table are
 // uploaded once per context and stay resident; a solve copies only the
 // temperature field and runs
-//   k_init_scalars -> k_tmax -> k_setup1 -> [k_grey_ib] -> k_setup2 ->
-//   k_levels -> k_patch_desc -> k_march -> k_tally_multi
+//   k_init_scalars -> k_tmax -> k_setup1 -> [k_grey_tables] -> k_setup2 ->
+//   k_levels -> k_march -> k_tally_multi
 // on the context's stream without any host synchronisation.
 #include <cuda_runtime.h>
 #include <stdio.h>
@@ -168,6 +168,12 @@ struct SlotCommon {
     DScalars *d_sc = nullptr, *h_sc = nullptr;
     double *d_partial = nullptr;
     size_t partial_cap = 0;
+    // the results, one block on the device: q64 | var64 | qw64 | vw64 (double),
+    // Qc | Sc | Wq | Ws (float); pinned staging of the whole block when it is
+    // small (h_all), else of the floats only
+    double *d_res = nullptr;
+    unsigned char *h_res = nullptr;
+    bool h_all = false;
     double *d_q64 = nullptr, *d_var64 = nullptr, *d_qw64 = nullptr, *d_vw64 = nullptr;
     float *d_Qc = nullptr, *d_Sc = nullptr, *d_Wq = nullptr, *d_Ws = nullptr;
     float *h_Qc = nullptr, *h_Sc = nullptr, *h_Wq = nullptr, *h_Ws = nullptr;
@@ -303,18 +309,8 @@ struct Impl : ImplBase {
             dfree(s.d_sc);
             hfree(s.h_sc);
             dfree(s.d_partial);
-            dfree(s.d_q64);
-            dfree(s.d_var64);
-            dfree(s.d_qw64);
-            dfree(s.d_vw64);
-            dfree(s.d_Qc);
-            dfree(s.d_Sc);
-            dfree(s.d_Wq);
-            dfree(s.d_Ws);
-            hfree(s.h_Qc);
-            hfree(s.h_Sc);
-            hfree(s.h_Wq);
-            hfree(s.h_Ws);
+            dfree(s.d_res);
+            hfree(s.h_res);
             dfree(s.d_counter);
             dfree(s.d_out);
             hfree(s.h_out);
@@ -367,6 +363,14 @@ struct Impl : ImplBase {
         if (!tmp.empty()) RC_CK(cudaMemcpy(dst, tmp.data(), tmp.size() * sizeof(T), cudaMemcpyHostToDevice));
         return RC_OK;
     }
+
+    // Results up to this size come back by one copy into pinned memory, doubles
+    // included, and are copied to the caller's arrays from there: a copy to
+    // pageable memory costs about 10 us of waiting, and rc_collect has up to
+    // four of them (16^3 grey: 321 -> 255 us a call with the merged set-up
+    // kernels).  Above it the extra pass
+    // over host memory would cost more than the waits.
+    static constexpr size_t kStageAll = (size_t)2 << 20;
 
     // Table coordinates of a level with its halo.
     long long level_cells(int l) const {
@@ -427,22 +431,24 @@ struct Impl : ImplBase {
             RC_CK(cudaHostAlloc((void **)&s.h_T, nfield * sizeof(float), cudaHostAllocDefault));
             RC_CK(cudaMalloc((void **)&s.d_sc, sizeof(DScalars)));
             RC_CK(cudaHostAlloc((void **)&s.h_sc, sizeof(DScalars), cudaHostAllocDefault));
-            RC_CK(cudaMalloc((void **)&s.d_q64, ncf * sizeof(double)));
-            RC_CK(cudaMalloc((void **)&s.d_var64, ncf * sizeof(double)));
-            RC_CK(cudaMalloc((void **)&s.d_qw64, nwc * sizeof(double)));
-            RC_CK(cudaMalloc((void **)&s.d_vw64, nwc * sizeof(double)));
-            RC_CK(cudaMalloc((void **)&s.d_Qc, ncf * sizeof(float)));
-            RC_CK(cudaMalloc((void **)&s.d_Sc, ncf * sizeof(float)));
-            RC_CK(cudaMalloc((void **)&s.d_Wq, nwc * sizeof(float)));
-            RC_CK(cudaMalloc((void **)&s.d_Ws, nwc * sizeof(float)));
-            RC_CK(cudaMemset(s.d_Wq, 0, nwc * sizeof(float)));
-            RC_CK(cudaMemset(s.d_Ws, 0, nwc * sizeof(float)));
-            RC_CK(cudaMemset(s.d_qw64, 0, nwc * sizeof(double)));
-            RC_CK(cudaMemset(s.d_vw64, 0, nwc * sizeof(double)));
-            RC_CK(cudaHostAlloc((void **)&s.h_Qc, ncf * sizeof(float), cudaHostAllocDefault));
-            RC_CK(cudaHostAlloc((void **)&s.h_Sc, ncf * sizeof(float), cudaHostAllocDefault));
-            RC_CK(cudaHostAlloc((void **)&s.h_Wq, nwc * sizeof(float), cudaHostAllocDefault));
-            RC_CK(cudaHostAlloc((void **)&s.h_Ws, nwc * sizeof(float), cudaHostAllocDefault));
+            const size_t nd = 2 * ncf + 2 * nwc, nf = nd;  // doubles, floats of the results
+            RC_CK(cudaMalloc((void **)&s.d_res, nd * sizeof(double) + nf * sizeof(float)));
+            RC_CK(cudaMemset(s.d_res, 0, nd * sizeof(double) + nf * sizeof(float)));
+            s.d_q64 = s.d_res;
+            s.d_var64 = s.d_q64 + ncf;
+            s.d_qw64 = s.d_var64 + ncf;
+            s.d_vw64 = s.d_qw64 + nwc;
+            s.d_Qc = reinterpret_cast<float *>(s.d_res + nd);
+            s.d_Sc = s.d_Qc + ncf;
+            s.d_Wq = s.d_Sc + ncf;
+            s.d_Ws = s.d_Wq + nwc;
+            s.h_all = nd * sizeof(double) + nf * sizeof(float) <= kStageAll;
+            RC_CK(cudaHostAlloc((void **)&s.h_res, (s.h_all ? nd * sizeof(double) : 0) + nf * sizeof(float),
+                                cudaHostAllocDefault));
+            s.h_Qc = reinterpret_cast<float *>(s.h_res + (s.h_all ? nd * sizeof(double) : 0));
+            s.h_Sc = s.h_Qc + ncf;
+            s.h_Wq = s.h_Sc + ncf;
+            s.h_Ws = s.h_Wq + nwc;
             RC_CK(cudaMalloc((void **)&s.d_counter, sizeof(unsigned long long)));
             RC_CK(cudaMalloc((void **)&s.d_out, sizeof(TallyOut)));
             RC_CK(cudaHostAlloc((void **)&s.h_out, sizeof(TallyOut), cudaHostAllocDefault));
@@ -857,7 +863,8 @@ struct Impl : ImplBase {
     }
 
     // Set-up kernels of one solve (everything before the march).
-    int enqueue_setup(Slot<R> &s, cudaStream_t st) {
+    // desc_dev: the descriptor on the device, copied there before.
+    int enqueue_setup(Slot<R> &s, DSolve<R> *desc_dev, cudaStream_t st) {
         std::string *err_ = &c->err;
         const rc_params &p = c->p;
         k_init_scalars<<<1, 32, 0, st>>>(s.d_sc);
@@ -865,16 +872,14 @@ struct Impl : ImplBase {
         int gb = (int)std::min<long long>((ncell + 255) / 256, (long long)c->num_sms * 8);
         k_tmax<<<std::max(gb, 1), 256, 0, st>>>(s.d_T, p.imax, p.jmax, p.kmax, s.d_sc);
         R *Tnb = p.grey ? s.d_Tnb_grey : d_Tnb;
-        k_setup1<R><<<1, 32, 0, st>>>(s.d_sc, Tnb, d_kP, nT, p.grey, p.Tmins, p.abscoeff, p.stefan, p.photmax,
+        k_setup1<R><<<1, 32, 0, st>>>(s.d_sc, desc_dev, Tnb, d_kP, nT, p.grey, p.Tmins, p.abscoeff, p.stefan, p.photmax,
                                       p.eps[RC_WEST], p.eps[RC_EAST]);
         const R *Ibt = d_Ibt;
         if (p.grey) {
             const int n = nT * nB;
-            k_grey_ib<R><<<std::max(1, std::min((n + 255) / 256, c->num_sms * 4)), 256, 0, st>>>(s.d_Ibt_grey, Tnb,
-                                                                                                  d_wvc, nT, nB);
+            k_grey_tables<R><<<std::max(1, std::min((n + 255) / 256, c->num_sms * 4)), 256, 0, st>>>(
+                s.d_Ibt_grey, s.d_ki_grey, d_kt, Tnb, d_wvc, nT, nB);
             Ibt = s.d_Ibt_grey;
-            k_build_ki<R><<<std::max(1, std::min((n + 255) / 256, c->num_sms * 4)), 256, 0, st>>>(s.d_ki_grey, d_kt,
-                                                                                                Ibt, nB, 1, nT);
         }
         k_setup2<R><<<1, 256, 0, st>>>(s.d_sc, s.d_cdf_f, s.d_cdf_s, s.d_guide_f, s.d_guide_s, s.d_den_f, s.d_ibm,
                                        d_prob, Ibt, d_kt, d_wvl, d_wvr, nT, nB, nQ, p.grey, p.calcwalls);
@@ -1053,15 +1058,11 @@ struct Impl : ImplBase {
         const size_t nfield = (size_t)(p.imax + 2) * (p.jmax + 2) * (p.kmax + 2);
         if (T_dev) RC_CK(cudaMemcpyAsync(s.d_T, T_dev, nfield * sizeof(float), cudaMemcpyDeviceToDevice, st));
         else if (!field_ready) RC_CK(cudaMemcpyAsync(s.d_T, s.h_T, nfield * sizeof(float), cudaMemcpyHostToDevice, st));
-        int rc = enqueue_setup(s, st);
-        if (rc) return rc;
         if (desc_dev == s.d_desc) {
             RC_CK(cudaMemcpyAsync(s.d_desc, s.h_desc, sizeof(DSolve<R>), cudaMemcpyHostToDevice, st));
             RC_CK(cudaMemcpyAsync(s.d_out, s.h_out, sizeof(TallyOut), cudaMemcpyHostToDevice, st));
         }
-        k_patch_desc<R><<<1, 32, 0, st>>>(desc_dev, s.d_sc);
-        RC_CK(cudaGetLastError());
-        return RC_OK;
+        return enqueue_setup(s, desc_dev, st);
     }
 
     // Everything up to the march on stream st: field copy, set-up kernels
@@ -1284,17 +1285,25 @@ struct Impl : ImplBase {
         RC_FAILPOINT("collect");
         const size_t ncf = (size_t)p.imax * p.jmax * c->kloc;
         const size_t nwc = (size_t)2 * p.jmax * c->kloc;
-        if (Q || sigma) {
-            RC_CK(cudaMemcpyAsync(s.h_Qc, s.d_Qc, ncf * sizeof(float), cudaMemcpyDeviceToHost, s.st));
-            RC_CK(cudaMemcpyAsync(s.h_Sc, s.d_Sc, ncf * sizeof(float), cudaMemcpyDeviceToHost, s.st));
-            RC_CK(cudaMemcpyAsync(s.h_Wq, s.d_Wq, nwc * sizeof(float), cudaMemcpyDeviceToHost, s.st));
-            RC_CK(cudaMemcpyAsync(s.h_Ws, s.d_Ws, nwc * sizeof(float), cudaMemcpyDeviceToHost, s.st));
+        const size_t nd = 2 * ncf + 2 * nwc;
+        const bool all = s.h_all && (q64 || var64 || qw64 || vw64);
+        if (all) {
+            RC_CK(cudaMemcpyAsync(s.h_res, s.d_res, nd * (sizeof(double) + sizeof(float)), cudaMemcpyDeviceToHost, s.st));
+        } else {
+            if (Q || sigma) RC_CK(cudaMemcpyAsync(s.h_Qc, s.d_Qc, nd * sizeof(float), cudaMemcpyDeviceToHost, s.st));
+            if (q64) RC_CK(cudaMemcpyAsync(q64, s.d_q64, ncf * sizeof(double), cudaMemcpyDeviceToHost, s.st));
+            if (var64) RC_CK(cudaMemcpyAsync(var64, s.d_var64, ncf * sizeof(double), cudaMemcpyDeviceToHost, s.st));
+            if (qw64) RC_CK(cudaMemcpyAsync(qw64, s.d_qw64, nwc * sizeof(double), cudaMemcpyDeviceToHost, s.st));
+            if (vw64) RC_CK(cudaMemcpyAsync(vw64, s.d_vw64, nwc * sizeof(double), cudaMemcpyDeviceToHost, s.st));
         }
-        if (q64) RC_CK(cudaMemcpyAsync(q64, s.d_q64, ncf * sizeof(double), cudaMemcpyDeviceToHost, s.st));
-        if (var64) RC_CK(cudaMemcpyAsync(var64, s.d_var64, ncf * sizeof(double), cudaMemcpyDeviceToHost, s.st));
-        if (qw64) RC_CK(cudaMemcpyAsync(qw64, s.d_qw64, nwc * sizeof(double), cudaMemcpyDeviceToHost, s.st));
-        if (vw64) RC_CK(cudaMemcpyAsync(vw64, s.d_vw64, nwc * sizeof(double), cudaMemcpyDeviceToHost, s.st));
         RC_CK(cudaStreamSynchronize(s.st));
+        if (all) {
+            const double *h = reinterpret_cast<const double *>(s.h_res);
+            if (q64) memcpy(q64, h, ncf * sizeof(double));
+            if (var64) memcpy(var64, h + ncf, ncf * sizeof(double));
+            if (qw64) memcpy(qw64, h + 2 * ncf, nwc * sizeof(double));
+            if (vw64) memcpy(vw64, h + 2 * ncf + nwc, nwc * sizeof(double));
+        }
         if (Q || sigma) scatter(s, Q, sigma);
         if (s.h_sc->status & 2) return set_err(err_, RC_E_RANGE, "temperature field contains non-finite values");
         return RC_OK;

@@ -55,9 +55,10 @@ static __global__ void k_tmax(const float *__restrict__ T, int imax, int jmax, i
 }
 
 // Scalars of the solve (mc_gpu_noint.cu:74, 820-826, 1362-1366;
-// read_tables.cpp:36-38, 102-110).  One warp.
+// read_tables.cpp:36-38, 102-110), and the run-time values of the descriptor
+// on the device.  One warp.
 template <typename R>
-__global__ void k_setup1(DScalars *sc, R *Tnb, const R *kP, int nT, int grey, float Tmins, float abscoeff,
+__global__ void k_setup1(DScalars *sc, DSolve<R> *d, R *Tnb, const R *kP, int nT, int grey, float Tmins, float abscoeff,
                          double stefan, int photmax, float eps_w, float eps_e) {
     const float Tmax_f = __uint_as_float(sc->tmax_bits);
     const R Tmax = (R)Tmax_f;
@@ -98,19 +99,11 @@ __global__ void k_setup1(DScalars *sc, R *Tnb, const R *kP, int nT, int grey, fl
     sc->T0 = (double)T0;
     sc->inv_dT = (double)inv_dT;
     sc->Pm = table_coord(Tmax, T0, inv_dT, nT);
-}
-
-// Copy the run-time values of a solve into its descriptor (after k_setup1,
-// before the march).
-template <typename R>
-__global__ void k_patch_desc(DSolve<R> *d, const DScalars *sc) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        d->Pm = sc->Pm;
-        d->Ibmax_f = (R)sc->Ibmax_f;
-        d->Ibmax_w0 = (R)sc->Ibmax_w[0];
-        d->Ibmax_w1 = (R)sc->Ibmax_w[1];
-        d->row = sc->row;
-    }
+    d->Pm = sc->Pm;
+    d->row = row;
+    d->Ibmax_f = (R)sc->Ibmax_f;
+    d->Ibmax_w0 = (R)sc->Ibmax_w[0];
+    d->Ibmax_w1 = (R)sc->Ibmax_w[1];
 }
 
 static __global__ void k_init_scalars(DScalars *sc) {
@@ -123,29 +116,22 @@ static __global__ void k_init_scalars(DScalars *sc) {
     }
 }
 
-// Interleaved k / I_b rows {k[t], Ib[t], k[t+1], Ib[t+1]} (last row repeated).
+// Grey gas: the Planck table I_b(Tnb[t], wvc[b]) (read_tables.cpp:140-148) and
+// the interleaved rows {k[t], Ib[t], k[t+1], Ib[t+1]} (last row repeated), one
+// thread per entry (the second Planck value of a row is cheaper than a second
+// launch that would read it).
 template <typename R>
-__global__ void k_build_ki(KIRow<R> *ki, const R *kt, const R *Ibt, int nB, int nQ, int nT) {
-    const int n = nB * nQ * nT;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const int t = e % nT, bg = e / nT, nb = bg / nQ;
-        const int t1 = min(t + 1, nT - 1);
-        KIRow<R> r;
-        r.k0 = kt[(size_t)bg * nT + t];
-        r.k1 = kt[(size_t)bg * nT + t1];
-        r.ib0 = Ibt[(size_t)nb * nT + t];
-        r.ib1 = Ibt[(size_t)nb * nT + t1];
-        ki[e] = r;
-    }
-}
-
-// Grey-gas Planck table I_b(Tnb[t], wvc[b]) (read_tables.cpp:140-148).
-template <typename R>
-__global__ void k_grey_ib(R *Ibt, const R *Tnb, const R *wvc, int nT, int nB) {
+__global__ void k_grey_tables(R *Ibt, KIRow<R> *ki, const R *kt, const R *Tnb, const R *wvc, int nT, int nB) {
     const int n = nT * nB;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-        const int b = e / nT, t = e % nT;
-        Ibt[e] = (R)rc_planck((double)Tnb[t], (double)wvc[b]);
+        const int b = e / nT, t = e % nT, t1 = min(t + 1, nT - 1);
+        KIRow<R> r;
+        r.k0 = kt[e];
+        r.k1 = kt[e - t + t1];
+        r.ib0 = (R)rc_planck((double)Tnb[t], (double)wvc[b]);
+        r.ib1 = (R)rc_planck((double)Tnb[t1], (double)wvc[b]);
+        Ibt[e] = r.ib0;
+        ki[e] = r;
     }
 }
 
@@ -340,7 +326,7 @@ __global__ void k_trace(const DSolve<R> *Sp, int n, const rc_bundle_id *ids, rc_
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     // the descriptor of a finished solve, its run-time fields patched by
-    // k_patch_desc before the march
+    // k_setup1 before the march
     const DSolve<R> &S = *Sp;
     const rc_bundle_id id = ids[t];
     rc_trace_rec rec;

@@ -894,15 +894,13 @@ int solve_noalloc_t(rc_ctx *c, const float *T_dev, int zstart, double *q64, doub
     cudaStream_t st = s.st;
     const size_t nfield = (size_t)(p.imax + 2) * (p.jmax + 2) * (p.kmax + 2);
     RC_CK(cudaMemcpyAsync(s.d_T, T_dev, nfield * sizeof(float), cudaMemcpyDeviceToDevice, st));
-    rc = im.enqueue_setup(s, st);
-    if (rc) return rc;
     im.fill_desc(s, zstart, rpt, *s.h_desc);
     s.h_desc->partial = scratch;
     if (!im.decomposition_fits(*s.h_desc))
         return set_err(err_, RC_E_INVALID, "too many work items for one solve: raise rays_per_thread");
     RC_CK(cudaMemcpyAsync(s.d_desc, s.h_desc, sizeof(DSolve<R>), cudaMemcpyHostToDevice, st));
-    k_patch_desc<R><<<1, 32, 0, st>>>(s.d_desc, s.d_sc);
-    RC_CK(cudaGetLastError());
+    rc = im.enqueue_setup(s, s.d_desc, st);
+    if (rc) return rc;
     TallyOut *o = s.h_out;
     o->q64 = q64;
     o->var64 = var64;
