@@ -19,8 +19,8 @@ namespace rc {
 //   * every lane traces one ray; the warp steps all its rays until at least
 //     kFeedIdle lanes are idle, then retires the rays that stopped and hands
 //     those lanes the next emitted bundles (warp ballot + prefix count);
-//   * two to four tiles can be in flight (tile_bufs): once every bundle of a tile has been
-//     emitted, the warp fetches the next tile and keeps
+//   * two or three tiles can be in flight (tile_bufs): once every bundle of a
+//     tile has been emitted, the warp fetches the next tile and keeps
 //     emitting from it while the last rays of earlier tiles finish, so long
 //     rays do not leave the other lanes idle;
 //   * each bundle's FP64 tally goes to its own shared-memory slot; when a
@@ -34,6 +34,13 @@ namespace rc {
 // temperature pyramid and the k / I_b tables (48-byte entries, an earlier
 // layout, were 1.2% slower; 64-byte entries 4%).  The scattering variant
 // keeps these entries and adds a small side array (see WarpShared).
+//
+// The kernel is bound by instruction issue (81-83% of the slots; DRAM idle):
+// on the 64^3 narrow-band channel 607 warp instructions per emitted wave,
+// about 330 per pass that retires and feeds, 120-140 per step-loop iteration
+// at 23-24 lanes.  With two tiles in flight, four divergent paths per
+// iteration and 64 registers it took 26.6 ms for photmax 256 there and 60 ms
+// on the 192x128x128 channel; now 22 and 30-32 ms.
 
 struct MarchArgs {
     const void *desc;            // DSolve<R> on the device (run-time fields patched)
@@ -173,11 +180,11 @@ __device__ __forceinline__ void flush_counters(DScalars *sc, unsigned long long 
 // Ring position of a running index (below 2 kRing).
 __device__ __forceinline__ int ring_at(int i) { return i < kRing ? i : i - kRing; }
 
-// MINB: resident 256-thread blocks per SM the register allocation must
-// allow (2: up to 128 registers, 3: 80, 4: 64).  SCAT: the variant for
-// media with scattering particles (solves without them run in it unchanged).
-// Registers of the variants (MINB, the occupancy knob): 64 lets four 256-thread
-// blocks onto an SM, 72 seven 128-thread blocks, 128 two 256-thread blocks.
+// SCAT: the variant for media with scattering particles.  MINB: the occupancy
+// knob.  Registers of its values: 128 lets two 256-thread blocks onto an SM, 72
+// seven 128-thread blocks, 64 four 256-thread blocks.  72 is the default: 28
+// warps and no more than 24 bytes of spill (64^3, photmax 256: 22.1 ms, with
+// 64 registers 24.2, with 80 and 24 warps 23.3).
 constexpr int march_regs(int minb) { return minb >= 4 ? 64 : minb == 3 ? 72 : 128; }
 
 template <typename R, int MINB, bool SCAT>
