@@ -265,6 +265,8 @@ typedef struct rc_solve_info {
     float Ibmax_fluid;     /* energy per fluid bundle */
     int   table_row;       /* table row nearest Tmax (mc_gpu_noint.cu:1110) */
     int   status;          /* bit 0: T outside table range, bit 1: non-finite T;
+                              bit 4: grey_nT > 256 and a temperature beyond row 255
+                              (collecting then fails with RC_E_RANGE);
                               bounds-checked build (libradchan_checked.so): bit 3 an
                               index was out of bounds, bits 8-15 the first such site */
     double bundles;        /* bundles traced */
@@ -338,7 +340,8 @@ int rc_autotune(rc_ctx *ctx, const float *T, int zstart, int pilot_photmax,
  * qw64/vw64 rows of a wall whose flux is not computed are set to 0.  With
  * no ticket to read rc_solve_info from, the solve's status word is reported
  * by the return code: RC_E_RANGE, with the outputs written, when T was not
- * finite (status bit 1), an index was out of bounds (bit 3, bounds-checked
+ * finite (status bit 1), a temperature lay beyond the 256th row of a longer
+ * grey table (bit 4), an index was out of bounds (bit 3, bounds-checked
  * build; the message names the site) or T lay outside the table range
  * (bit 0, end rows used); rc_last_error says which. */
 int rc_solve_noalloc(rc_ctx *ctx, const float *T_dev, int zstart, double *q64_dev, double *var64_dev,

@@ -71,7 +71,8 @@ struct alignas(4 * sizeof(R)) KIRow {
 struct DScalars {
     unsigned int tmax_bits;   // float bits of max T (non-negative)
     unsigned int tmin_bits;   // float bits of min T
-    int status;               // bit 0 out of table, bit 1 non-finite, bit 2 T <= 0, bit 3 index out of bounds
+    int status;               // bit 0 out of table, bit 1 non-finite, bit 2 T <= 0, bit 3 index out of bounds,
+                              // bit 4 a coordinate beyond 16 bits (cell_coord)
     int tm, row;
     int bad_site;             // first out-of-bounds site (bounds-checked build)
     double Tmax, kappamax, Ibmax_f, Ibmax_w[2];
@@ -194,7 +195,7 @@ template <> struct RT<double> {
 
 // Table coordinate of a temperature with 8 fractional bits, the weight
 // precision of the texture unit the reference interpolates with:
-// q = rint(256 * clamp((T - T0)/dT, 0, nT-1)); NaN -> 0.  nT <= 256.
+// q = rint(256 * clamp((T - T0)/dT, 0, nT-1)); NaN -> 0.
 template <typename R>
 __device__ __forceinline__ int table_coord(R T, R T0, R inv_dT, int nT) {
     const R p = RT<R>::fmin_(RT<R>::fmax_((T - T0) * inv_dT, (R)0), (R)(nT - 1));
@@ -358,13 +359,23 @@ struct Ray {
     double De;
 };
 // Coordinates of the halo cells around every level say what the wall between
-// does with a ray (256 table rows end at 65280): reflect it, let it re-enter
-// through the opposite face, or end it (kBlack + wall: black walls, and any
-// other type, whose rays are lost).
-constexpr int kSpecular = 0xfff0, kPeriodic = 0xfff1, kBlack = 0xfff8;
+// does with a ray: reflect it, let it re-enter through the opposite face, or
+// end it (kBlack + wall: black walls, and any other type, whose rays are
+// lost).  256 table rows end at 65280; a grey table may have more, and a cell
+// that lies among its further rows must not read as a wall (cell_coord).
+constexpr int kSpecular = 0xfff8, kPeriodic = 0xfff9, kBlack = 0xfffa;
 
 __host__ __device__ __forceinline__ int halo_code(int wtype, int w) {
     return wtype == 1 ? kPeriodic : wtype == 3 ? kSpecular : kBlack + w;
+}
+
+// A coordinate as the 16-bit arrays hold it: the cells' below the halo codes,
+// the walls' of all 16 bits.  One above (a grey table of more than 256 rows,
+// a hot cell) is cut to the largest and reported (bit 4 of the status word).
+__host__ __device__ __forceinline__ uint16_t cell_coord(int q, bool wall, bool &cut) {
+    const int most = wall ? 0xffff : kSpecular - 1;
+    cut = q > most;
+    return (uint16_t)(cut ? most : q);
 }
 
 // Philox counter of one bundle: (h, v | kind << 24, cell, 0).

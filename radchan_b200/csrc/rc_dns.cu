@@ -329,7 +329,7 @@ int rc_dns_source(rc_ctx *c, rc_ticket t, const rc_dns_coupling *cfg, const doub
     const int status = s.h_sc->status;
     s.state = 0;
     s.ticket = -1;
-    if (status & 2) return set_err(err_, RC_E_RANGE, "temperature field contains non-finite values");
+    if (const char *bad = status_error(status)) return set_err(err_, RC_E_RANGE, bad);
     return RC_OK;
 }
 

@@ -142,6 +142,13 @@ __global__ void k_tally_multi(const DSolve<R> *solves, const TallyOut *outs) {
     }
 }
 
+// Status bits (DScalars::status) after which a solve's results are no answer.
+inline const char *status_error(int status) {
+    if (status & 2) return "temperature field contains non-finite values";
+    if (status & 16) return "a temperature lies beyond the 256 table rows that the cells' coordinates reach: lower grey_nT";
+    return nullptr;
+}
+
 struct ImplBase {
     virtual ~ImplBase() {}
 };
@@ -1305,7 +1312,7 @@ struct Impl : ImplBase {
             if (vw64) memcpy(vw64, h + 2 * ncf + nwc, nwc * sizeof(double));
         }
         if (Q || sigma) scatter(s, Q, sigma);
-        if (s.h_sc->status & 2) return set_err(err_, RC_E_RANGE, "temperature field contains non-finite values");
+        if (const char *bad = status_error(s.h_sc->status)) return set_err(err_, RC_E_RANGE, bad);
         return RC_OK;
     }
 
@@ -1320,7 +1327,7 @@ struct Impl : ImplBase {
         const size_t ncf = (size_t)c->p.imax * c->p.jmax * c->kloc;
         const size_t nwc = (size_t)2 * c->p.jmax * c->kloc;
         scatter_from(pack, pack + ncf, pack + 2 * ncf, pack + 2 * ncf + nwc, Q, sigma);
-        if (s.h_sc->status & 2) return set_err(err_, RC_E_RANGE, "temperature field contains non-finite values");
+        if (const char *bad = status_error(s.h_sc->status)) return set_err(err_, RC_E_RANGE, bad);
         return RC_OK;
     }
     size_t packed_floats() const {
@@ -1377,7 +1384,7 @@ struct Impl : ImplBase {
         RC_CK(cudaStreamSynchronize(s.st));
         s.state = 0;
         s.ticket = -1;
-        if (s.h_sc->status & 2) return set_err(err_, RC_E_RANGE, "temperature field contains non-finite values");
+        if (const char *bad = status_error(s.h_sc->status)) return set_err(err_, RC_E_RANGE, bad);
         return RC_OK;
     }
 

@@ -261,9 +261,10 @@ struct LevelJobs {
 
 template <typename R>
 __global__ void k_levels(const float *__restrict__ T, int imax, int jmax, int kmax, LevelJobs jobs,
-                         const DScalars *sc, int nT) {
+                         DScalars *sc, int nT) {
     const int nx = imax + 2, ny = jmax + 2, nz = kmax + 2;
     const R T0 = (R)sc->T0, inv_dT = (R)sc->inv_dT;
+    bool cut, any_cut = false;
     for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < jobs.total;
          e += (long long)gridDim.x * blockDim.x) {
         int jb = 0;
@@ -292,7 +293,8 @@ __global__ void k_levels(const float *__restrict__ T, int imax, int jmax, int km
             const float t1 = ((float)ic - 0.5f) * rxf + 1.0f;
             const float t2 = ((float)jc - 0.5f) * ryf + 1.0f;
             const float t3 = ((float)kc - 0.5f) * rzf + 1.0f;
-            dst[l] = (uint16_t)table_coord((R)tex_sample(T, nx, ny, nz, t1, t2, t3), T0, inv_dT, nT);
+            dst[l] = cell_coord(table_coord((R)tex_sample(T, nx, ny, nz, t1, t2, t3), T0, inv_dT, nT), false, cut);
+            any_cut |= cut;
         } else {
             const int w = J.type - 1;
             float x, y, z;
@@ -312,9 +314,11 @@ __global__ void k_levels(const float *__restrict__ T, int imax, int jmax, int km
                 y = ((float)jc - 0.5f) * ryf + 1.0f;
                 z = (w == RC_BOT) ? (J.face ? 1.0f : 1.5f) : (J.face ? (float)kmax + 1.0f : (float)kmax + 0.5f);
             }
-            dst[l] = (uint16_t)table_coord((R)tex_sample(T, nx, ny, nz, x, y, z), T0, inv_dT, nT);
+            dst[l] = cell_coord(table_coord((R)tex_sample(T, nx, ny, nz, x, y, z), T0, inv_dT, nT), true, cut);
+            any_cut |= cut;
         }
     }
+    if (any_cut) atomicOr(&sc->status, 16);
 }
 
 // ---------------------------------------------------------------------------

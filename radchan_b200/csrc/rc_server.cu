@@ -463,8 +463,8 @@ void finish_stage(rc_server *sv, SrvReq *r) {
     Impl<float> &im = *static_cast<Impl<float> *>(r->ctx->impl);
     Slot<float> &s = *r->slot;
     const size_t ncf = (size_t)r->p.imax * r->p.jmax * r->ctx->kloc;
-    if (s.h_sc->status & 2) {
-        fail(sv, r, RC_E_RANGE, "temperature field contains non-finite values");
+    if (const char *bad = status_error(s.h_sc->status)) {
+        fail(sv, r, RC_E_RANGE, bad);
         return;
     }
     if (r->stage == ST_PILOT) {

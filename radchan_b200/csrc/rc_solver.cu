@@ -927,7 +927,8 @@ int solve_noalloc_t(rc_ctx *c, const float *T_dev, int zstart, double *q64, doub
     // solve travels in the return code and the message.  The outputs are
     // written in every case below.
     const int status = s.h_sc->status;
-    if (status & 2) return set_err(err_, RC_E_RANGE, "temperature field contains non-finite values (status bit 1)");
+    if (const char *bad = status_error(status))
+        return set_err(err_, RC_E_RANGE, std::string(bad) + (status & 2 ? " (status bit 1)" : " (status bit 4)"));
     if (status & 8)
         return set_err(err_, RC_E_RANGE,
                        "an index was out of bounds in the march (status bit 3, bounds-checked build), first at site " +

@@ -1,0 +1,39 @@
+// Integer rules that the march's kernels share with the host, checked without
+// a GPU: prints one "ok <name>" line per rule (tests/test_cpu_device_rules.py).
+#include <stdio.h>
+#include "radchan.h"
+#include "rc_device.cuh"
+
+using namespace rc;
+
+static int fail(const char *what, long long at) {
+    printf("bad %s at %lld\n", what, at);
+    return 1;
+}
+
+// A cell's coordinate never reads as a wall, for any number of table rows;
+// those below the codes are stored as they are, the others are reported.
+static int coords() {
+    for (int w = 0; w < 6; ++w)
+        for (int t = 0; t <= 6; ++t) {
+            const int code = halo_code(t, w);
+            if (code < kSpecular || code > 0xffff) return fail("halo code", code);
+            if (t != 1 && t != 3 && (code < kBlack || code - kBlack != w)) return fail("wall of a code", code);
+        }
+    if (kPeriodic >= kBlack || kSpecular >= kBlack || 255 * 256 >= kSpecular) return fail("order of the codes", 0);
+    for (int q = 0; q <= 1000 * 256; ++q) {
+        bool cut_c, cut_w;
+        const int c = cell_coord(q, false, cut_c), wv = cell_coord(q, true, cut_w);
+        if (c >= kSpecular) return fail("cell reads as a wall", q);
+        if (cut_c ? q < kSpecular : c != q) return fail("cell coordinate", q);
+        if (cut_w ? q <= 0xffff : wv != q) return fail("wall coordinate", q);
+    }
+    printf("ok coords\n");
+    return 0;
+}
+
+int main() {
+    int bad = 0;
+    bad |= coords();
+    return bad;
+}
