@@ -322,12 +322,18 @@ __device__ __forceinline__ void select_band_g(const DSolve<R> &S, int row, int k
     if (wall) g = S.nQ > 1 ? bisect(S.probq, S.nQ, u_g) : 0;
 }
 
+// The i and j of a cell in one word, 16 bits each.
+__host__ __device__ __forceinline__ unsigned pack_ij(int i, int j) { return (unsigned)i | (unsigned)j << 16; }
+__host__ __device__ __forceinline__ int unpack_i(unsigned ij) { return (int)(ij & 0xffffu); }
+__host__ __device__ __forceinline__ int unpack_j(unsigned ij) { return (int)(ij >> 16); }
+
 // A bundle after emission, placed at its start point: position, cell,
-// direction, sampled band/g and OERM weights.
+// direction, sampled band/g and OERM weights.  The edges, bands and g points
+// that the packed words hold are the limits of params_validate.
 template <typename R>
 struct alignas(16) Emitted {
     R sx, sy, sz, ratioI, invTi4;
-    int ij;    // ic | jc << 16: the emitting cell (fluid) or wall cell
+    unsigned ij;  // ic | jc << 16: the emitting cell (fluid) or wall cell
     int kk;    // kc | kind << 16 | pool index << 18 | pool parity << 29
     int nbg;   // nb | g << 20
 };
@@ -429,7 +435,7 @@ __device__ __forceinline__ bool emit_bundle(Emitted<R> &e, const DSolve<R> &S, i
                         : S.Pall[RC_IX(S.lva[0].y + cell_index(i, j, k, S.imax, S.jmax), S.n_P, SITE_EMIT_T, S)];
     const int ic = wall ? (east ? S.imax : 1) : i;
     e.nbg = nb | (g << 20);
-    e.ij = ic | (j << 16);
+    e.ij = pack_ij(ic, j);
     e.kk = k | (kind << 16);
     // OERM weights
     const KIRow<R> ki =
@@ -472,7 +478,7 @@ __device__ __forceinline__ void set_cell(Ray<R> &r, const DSolve<R> &S, const in
 template <typename R>
 __device__ __forceinline__ void place_bundle(Ray<R> &r, const DSolve<R> &S, const DSolve<R> &D, const Emitted<R> &e) {
     const int kind = (e.kk >> 16) & 3;
-    int ic = e.ij & 0xffff, jc = e.ij >> 16, kc = e.kk & 0xffff;
+    int ic = unpack_i(e.ij), jc = unpack_j(e.ij), kc = e.kk & 0xffff;
     // start point: the cell centre, or the wall cell's point on the wall
     // (kernel_fluid :117-122, kernel_surface :1381-1384)
     r.xp = kind == 0 ? S.xc[RC_IX(ic, S.imax + 2, SITE_CENTRE, S)] : (kind == 1 ? (R)0 : S.Lx);

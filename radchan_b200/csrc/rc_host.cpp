@@ -95,6 +95,9 @@ int params_validate(const rc_params &p, std::string &err) {
         return RC_E_INVALID;
     };
     if (p.imax < 1 || p.jmax < 1 || p.kmax < 1) return bad("imax, jmax, kmax must be >= 1");
+    // an emitted bundle keeps its cell in 16 bits an axis, its band in 20 and its
+    // g point in 11 (Emitted, rc_device.cuh)
+    if (p.imax > 65535 || p.jmax > 65535 || p.kmax > 65535) return bad("imax, jmax, kmax must be <= 65535");
     if (p.num_gpu != 1) return bad("num_gpu must be 1: one solve runs on one GPU");
     if (p.p_col < 1 || p.kmax % p.p_col != 0) return bad("p_col must divide kmax");
     if (p.grid_num < 1 || p.grid_num > RC_MAX_LEVELS) return bad("grid_num must be in [1, 9]");
@@ -121,6 +124,10 @@ int params_validate(const rc_params &p, std::string &err) {
     } else {
         if (p.nT < 2 || p.nB < 1 || p.nQ < 1) return bad("nT >= 2, nB >= 1, nQ >= 1 required");
     }
+    const int nB = p.grey ? p.grey_nB : p.nB, nQ = p.grey ? 1 : p.nQ, nT = p.grey ? p.grey_nT : p.nT;
+    if (nB > (1 << 20)) return bad("at most 1048576 bands");
+    if (nQ > (1 << 11)) return bad("at most 2048 g points");
+    if ((long long)nB * nQ * nT > 0x7fffffffLL) return bad("tables too large for 32-bit row offsets");
     if (p.floatpoint != 0 && p.floatpoint != 1) return bad("floatpoint must be 0 or 1");
     // 2 * 1 bits of kind and 24 bits of replicate in the Philox counter
     if (p.nVar > (1 << 24)) return bad("nVar too large");

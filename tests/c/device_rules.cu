@@ -32,8 +32,21 @@ static int coords() {
     return 0;
 }
 
+// The cell of an emitted bundle, for every edge that params_validate accepts.
+static int packing() {
+    const int some[] = {0, 1, 2, 255, 256, 32766, 32767, 32768, 32769, 65534, 65535};
+    for (int j = 0; j <= 65535; ++j)
+        for (int i : some) {
+            const unsigned a = pack_ij(i, j), b = pack_ij(j, i);
+            if (unpack_i(a) != i || unpack_j(a) != j || unpack_i(b) != j || unpack_j(b) != i) return fail("packing", j);
+        }
+    printf("ok packing\n");
+    return 0;
+}
+
 int main() {
     int bad = 0;
     bad |= coords();
+    bad |= packing();
     return bad;
 }

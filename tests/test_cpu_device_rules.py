@@ -1,12 +1,15 @@
 """Integer rules of the device code that decide whether an access stays in
 bounds, compiled for the host and run over their ranges (tests/c/device_rules.cu):
-a cell's table coordinate against the codes of the halo."""
+a cell's table coordinate against the codes of the halo, and an emitted
+bundle's packed cell, whose limits the parameter check keeps."""
 import os
 import subprocess
 
 import pytest
 
+from radchan_b200 import api
 from radchan_b200 import build as B
+from radchan_b200 import workloads as W
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 
@@ -22,6 +25,27 @@ def rules(tmp_path_factory):
     return r.stdout
 
 
-@pytest.mark.parametrize("name", ["coords"])
+@pytest.mark.parametrize("name", ["coords", "packing"])
 def test_rule_holds(rules, name):
     assert "ok " + name in rules.splitlines(), rules
+
+
+@pytest.mark.parametrize("axis", ["imax", "jmax", "kmax"])
+def test_edges_beyond_the_packed_cell_are_refused(axis):
+    at = ["imax", "jmax", "kmax"].index(axis)
+    for edge, ok in ((32767, True), (32768, True), (65535, True), (65536, False), (131072, False)):
+        n = [4, 4, 4]
+        n[at] = edge
+        msg = api.validate(W.channel_params(*n, grey=True))
+        assert (msg == "") == ok, (edge, msg)
+        assert ok or axis in msg
+
+
+def test_table_dimensions_beyond_the_packed_band_are_refused():
+    for kw, ok in ((dict(nB=1 << 20, nQ=1, nT=2), True), (dict(nB=(1 << 20) + 1, nQ=1, nT=2), False),
+                   (dict(nB=2, nQ=2048, nT=2), True), (dict(nB=2, nQ=2049, nT=2), False),
+                   (dict(nB=32767, nQ=256, nT=256), True), (dict(nB=32768, nQ=256, nT=256), False)):
+        assert (api.validate(W.channel_params(8, 8, 8, **kw)) == "") == ok, kw
+    p = W.channel_params(8, 8, 8, grey=True)
+    p.grey_nB = (1 << 20) + 1
+    assert "bands" in api.validate(p)
