@@ -244,11 +244,12 @@ __device__ __forceinline__ R coord_frac(int q) {
 }
 
 // Offset of cell (i,j,k) (1-based) of a level of im x jm cells per plane, i
-// fastest, one halo cell on every side (halo_code).
+// fastest, one halo cell on every side (halo_code).  The offsets of all levels
+// together fit 32 bits without a sign (params_validate).
 // (A 4x4x4-brick layout was measured 2-3% slower: its index arithmetic
 // costs more issue slots than its locality saves in L1 misses.)
-__host__ __device__ __forceinline__ int cell_index(int i, int j, int k, int im, int jm) {
-    return i + (im + 2) * (j + (jm + 2) * k);
+__host__ __device__ __forceinline__ unsigned cell_index(int i, int j, int k, int im, int jm) {
+    return i + (unsigned)(im + 2) * (j + (unsigned)(jm + 2) * k);
 }
 
 // Linear interpolation in temperature along one table column at a clamped
@@ -357,7 +358,8 @@ struct Ray {
     R fx;
     int fi;
     float fj, fk, dy, dz;
-    int cidx, dx, dj, dk; // cell offset in Pall, offsets of the neighbours through the exit faces
+    unsigned cidx;        // cell offset in Pall
+    int dx, dj, dk;       // offsets of the neighbours through the exit faces
     int q;                // coordinate of the cell, the halo code beyond a wall
     int kio;              // first table row of the bundle's band and g point
     int ln;               // band | level << 20
@@ -432,7 +434,7 @@ __device__ __forceinline__ bool emit_bundle(Emitted<R> &e, const DSolve<R> &S, i
     int nb, g;
     select_band_g(S, row, kind, u_b, u_g, nb, g);
     const int Pi = wall ? S.Pw0[east][RC_IX(jk, (long long)S.kmax * S.jmax, SITE_WALL_EMIT_T, S)]
-                        : S.Pall[RC_IX(S.lva[0].y + cell_index(i, j, k, S.imax, S.jmax), S.n_P, SITE_EMIT_T, S)];
+                        : S.Pall[RC_IX((unsigned)S.lva[0].y + cell_index(i, j, k, S.imax, S.jmax), S.n_P, SITE_EMIT_T, S)];
     const int ic = wall ? (east ? S.imax : 1) : i;
     e.nbg = nb | (g << 20);
     e.ij = pack_ij(ic, j);
@@ -460,7 +462,7 @@ __device__ __forceinline__ void set_cell(Ray<R> &r, const DSolve<R> &S, const in
 #endif
     const int sj = A.z + 2, sk = sj * (A.w + 2);
     const bool nx = r.sx < (R)0, ny = r.sy < (R)0, nz = r.sz < (R)0;
-    r.cidx = A.y + c.x + sj * c.y + sk * c.z;
+    r.cidx = (unsigned)A.y + c.x + (unsigned)sj * c.y + (unsigned)sk * c.z;
     r.q = __ldg(S.Pall + RC_IX(r.cidx, S.n_P, SITE_PYRAMID, S));
     r.fi = A.x + c.x - (int)nx;
     r.fx = __ldg(S.faces + RC_IX(r.fi, S.n_faces, SITE_FACE, S));
@@ -611,17 +613,17 @@ __device__ __forceinline__ void wrap_cell(Ray<R> &r, const DSolve<R> &S) {
         const bool hi = r.fj > 0.f;
         r.yp = hi ? (R)0 : S.Ly;
         r.fj = hi ? 1.f : fjm - 1.f;
-        r.cidx -= A.w * r.dj;
+        r.cidx -= (unsigned)A.w * r.dj;
     } else if (r.fk < 0.f || r.fk > fkm) {
         const bool hi = r.fk > 0.f;
         r.zp = hi ? (R)0 : S.Lz;
         r.fk = hi ? 1.f : fkm - 1.f;
-        r.cidx -= km * r.dk;
+        r.cidx -= (unsigned)km * r.dk;
     } else {
         const bool hi = r.dx > 0;
         r.xp = hi ? (R)0 : S.Lx;
         r.fi = A.x + (hi ? 1 : A.z - 1);
-        r.cidx -= A.z * r.dx;
+        r.cidx -= (unsigned)A.z * r.dx;
         r.fx = __ldg(S.faces + RC_IX(r.fi, S.n_faces, SITE_FACE, S));
     }
     r.q = __ldg(S.Pall + RC_IX(r.cidx, S.n_P, SITE_PYRAMID, S));

@@ -111,6 +111,13 @@ int params_validate(const rc_params &p, std::string &err) {
             return bad("each level must divide the previous one (param.h:26)");
         if (p.maxs[l] < 0) return bad("maxs must be >= 0");
     }
+    // a ray's cell is an unsigned 32-bit offset into all levels with their halos
+    long long cells = 0, halo = 0;
+    for (int l = 0; l < p.grid_num; ++l) {
+        cells += (long long)p.maxi[l] * p.maxj[l] * p.maxk[l];
+        halo += (p.maxi[l] + 2LL) * (p.maxj[l] + 2LL) * (p.maxk[l] + 2LL);
+    }
+    if (cells > 0x7fffffffLL || halo > 0xffffffffLL) return bad("grid too large for 32-bit level offsets");
     if (p.maxs[p.grid_num - 1] < 1) return bad("the last level needs maxs >= 1");
     if (p.nVar < 1) return bad("nVar must be >= 1");
     if (p.photmax < 1) return bad("photmax must be >= 1");

@@ -257,7 +257,8 @@ struct Impl : ImplBase {
     rc_ctx *c = nullptr;
     R *d_faces = nullptr;              // every level's xu | yu | zu (one allocation)
     std::vector<R *> d_xu, d_yu, d_zu; // per-level views into d_faces
-    std::vector<int> face_off, lev_off;  // per-level offsets in d_faces / Slot::d_levAll
+    std::vector<int> face_off;       // per-level offsets in d_faces
+    std::vector<unsigned> lev_off;   // and in Slot::d_levAll
     long long n_faces = 0, n_pyramid = 0;  // their lengths
     R *d_xc = nullptr, *d_yc = nullptr, *d_zc = nullptr;
     R *d_kt = nullptr, *d_Ibt = nullptr, *d_probg = nullptr, *d_prob = nullptr, *d_probq = nullptr;
@@ -405,9 +406,8 @@ struct Impl : ImplBase {
                 faces.insert(faces.end(), g.xu.begin(), g.xu.end());
                 faces.insert(faces.end(), g.yu.begin(), g.yu.end());
                 faces.insert(faces.end(), g.zu.begin(), g.zu.end());
-                lev_off[l] = (int)po;
+                lev_off[l] = (unsigned)po;  // params_validate: the whole pyramid fits
                 po += level_cells(l);
-                if (po > 0x7fffffffLL) return set_err(err_, RC_E_INVALID, "grid too large for 32-bit level offsets");
             }
             faces.push_back(0.f);
             n_faces = (long long)faces.size();
@@ -746,7 +746,7 @@ struct Impl : ImplBase {
             int dy, dz;
             memcpy(&dy, &c->grid[l].dy, 4);
             memcpy(&dz, &c->grid[l].dz, 4);
-            d.lva[l] = make_int4(face_off[l], lev_off[l], L.im, L.jm);
+            d.lva[l] = make_int4(face_off[l], (int)lev_off[l], L.im, L.jm);
             d.lvb[l] = make_int4(L.km, L.maxs, dy, dz);
             for (int w = 0; w < 6; ++w) L.Pw[w] = s.d_lw[l][w];
             d.steps_to[l] = (l ? d.steps_to[l - 1] : 0) + p.maxs[l];

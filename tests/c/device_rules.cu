@@ -44,8 +44,27 @@ static int packing() {
     return 0;
 }
 
+// Offsets of cells in a pyramid of almost 2^32 entries, halo included.
+static int offsets() {
+    const int dims[][3] = {{1289, 1289, 1289}, {65535, 16380, 2}, {2, 30000, 35000}, {1, 1, 65535}, {1023, 1023, 1023}};
+    for (auto &n : dims) {
+        const int im = n[0], jm = n[1], km = n[2];
+        const int is[] = {0, 1, im, im + 1}, js[] = {0, 1, jm, jm + 1}, ks[] = {0, 1, km, km + 1};
+        for (int i : is)
+            for (int j : js)
+                for (int k : ks) {
+                    const long long want = i + (im + 2LL) * (j + (jm + 2LL) * k);
+                    if (want > 0xffffffffLL) return fail("the grid itself", want);
+                    if ((long long)cell_index(i, j, k, im, jm) != want) return fail("offset", want);
+                }
+    }
+    printf("ok offsets\n");
+    return 0;
+}
+
 int main() {
     int bad = 0;
+    bad |= offsets();
     bad |= coords();
     bad |= packing();
     return bad;

@@ -1,7 +1,8 @@
 """Integer rules of the device code that decide whether an access stays in
 bounds, compiled for the host and run over their ranges (tests/c/device_rules.cu):
 a cell's table coordinate against the codes of the halo, and an emitted
-bundle's packed cell, whose limits the parameter check keeps."""
+bundle's packed cell and the offset of a cell in a large pyramid, whose limits
+the parameter check keeps."""
 import os
 import subprocess
 
@@ -25,7 +26,7 @@ def rules(tmp_path_factory):
     return r.stdout
 
 
-@pytest.mark.parametrize("name", ["coords", "packing"])
+@pytest.mark.parametrize("name", ["coords", "offsets", "packing"])
 def test_rule_holds(rules, name):
     assert "ok " + name in rules.splitlines(), rules
 
@@ -49,3 +50,15 @@ def test_table_dimensions_beyond_the_packed_band_are_refused():
     p = W.channel_params(8, 8, 8, grey=True)
     p.grey_nB = (1 << 20) + 1
     assert "bands" in api.validate(p)
+
+
+def test_the_largest_grids_are_those_whose_pyramid_has_32_bit_offsets():
+    for n, ok in (((1289, 1289, 1289), True), ((1290, 1290, 1290), True), ((1291, 1291, 1291), False),
+                  ((30000, 35000, 2), True), ((30000, 36000, 2), False), ((65535, 32767, 1), False),
+                  ((1, 1, 65535), True)):
+        msg = api.validate(W.channel_params(*n, grey=True))
+        assert (msg == "") == ok, (n, msg)
+    lv = [(1200, 1200, 1200), (600, 600, 600), (300, 300, 300)]
+    assert api.validate(W.channel_params(*lv[0], grey=True, levels=lv, maxs=[5, 5, 100])) == ""
+    lv = [(1280, 1280, 1280), (640, 640, 640), (320, 320, 320)]
+    assert "32-bit" in api.validate(W.channel_params(*lv[0], grey=True, levels=lv, maxs=[5, 5, 100]))
