@@ -93,7 +93,8 @@ struct TallyOut {
 
 // Replicate sums -> per-cell mean and variance of the mean
 // (kernel_fluid :229-239, kernel_surface :1468-1478), into compact FP64 and
-// FP32 outputs; one solve per blockIdx.y.
+// FP32 outputs; one solve per blockIdx.y.  The rows of a wall whose flux is
+// not computed become 0 here, in the order of the solve's own stream.
 template <typename R>
 __global__ void k_tally_multi(const DSolve<R> *solves, const TallyOut *outs) {
     const int s = blockIdx.y;
@@ -138,6 +139,18 @@ __global__ void k_tally_multi(const DSolve<R> *solves, const TallyOut *outs) {
             if (o.vw64) o.vw64[off] = var;
             o.Wq[off] = (float)mean;
             o.Ws[off] = (float)sqrt(var);
+        }
+    }
+    if (S.nwalls < 2) {
+        const long long nwc = (long long)S.jmax * S.kloc;
+        const int w0 = S.nwalls ? 1 - S.wall_id[0] : 0, nw = 2 - S.nwalls;
+        for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < nw * nwc;
+             c += (long long)gridDim.x * blockDim.x) {
+            const long long off = w0 * nwc + c;
+            if (o.qw64) o.qw64[off] = 0.0;
+            if (o.vw64) o.vw64[off] = 0.0;
+            o.Wq[off] = 0.f;
+            o.Ws[off] = 0.f;
         }
     }
 }
@@ -440,7 +453,9 @@ struct Impl : ImplBase {
             RC_CK(cudaHostAlloc((void **)&s.h_sc, sizeof(DScalars), cudaHostAllocDefault));
             const size_t nd = 2 * ncf + 2 * nwc, nf = nd;  // doubles, floats of the results
             RC_CK(cudaMalloc((void **)&s.d_res, nd * sizeof(double) + nf * sizeof(float)));
-            RC_CK(cudaMemset(s.d_res, 0, nd * sizeof(double) + nf * sizeof(float)));
+            // (nothing is cleared here: a memset on the default stream is not
+            // ordered with a solve on the context's, a batch's or a server's
+            // streams; every solve writes all that it or a collect reads)
             s.d_q64 = s.d_res;
             s.d_var64 = s.d_q64 + ncf;
             s.d_qw64 = s.d_var64 + ncf;
@@ -465,7 +480,6 @@ struct Impl : ImplBase {
             s.d_levT.assign(nl, nullptr);
             {
                 RC_CK(cudaMalloc((void **)&s.d_levAll, n_pyramid * sizeof(uint16_t)));
-                RC_CK(cudaMemset(s.d_levAll, 0, n_pyramid * sizeof(uint16_t)));
                 for (int l = 0; l < nl; ++l) s.d_levT[l] = s.d_levAll + lev_off[l];
             }
             LevelJobs &J = s.jobs;
@@ -514,7 +528,6 @@ struct Impl : ImplBase {
             RC_CK(cudaMalloc((void **)&s.d_ibm, nBmax * sizeof(R)));
             RC_CK(cudaMalloc((void **)&s.d_guide_f, kGuide * sizeof(int)));
             RC_CK(cudaMalloc((void **)&s.d_guide_s, kGuide * sizeof(int)));
-            RC_CK(cudaMemset(s.d_guide_s, 0, kGuide * sizeof(int)));
             if (p.grey) {
                 RC_CK(cudaMalloc((void **)&s.d_Tnb_grey, p.grey_nT * sizeof(R)));
                 RC_CK(cudaMalloc((void **)&s.d_Ibt_grey, (size_t)p.grey_nT * p.grey_nB * sizeof(R)));

@@ -211,7 +211,7 @@ __global__ void k_setup2(const DScalars *sc, R *cdf_f, R *cdf_s, int *guide_f, i
     for (int q = threadIdx.x; q < kGuide; q += blockDim.x) {
         const R x = (R)q / (R)kGuide;
         guide_f[q] = first_above(cdf_f, nB, x);
-        if (walls) guide_s[q] = first_above(cdf_s, nB, x);
+        guide_s[q] = walls ? first_above(cdf_s, nB, x) : 0;
     }
 }
 

@@ -911,12 +911,6 @@ int solve_noalloc_t(rc_ctx *c, const float *T_dev, int zstart, double *q64, doub
     o->Wq = s.d_Wq;
     o->Ws = s.d_Ws;
     RC_CK(cudaMemcpyAsync(s.d_out, s.h_out, sizeof(TallyOut), cudaMemcpyHostToDevice, st));
-    // The tally writes only the walls whose flux is computed; the others read
-    // 0, as the allocating entry points return them.
-    const int nwalls = s.h_desc->nwalls;
-    const size_t wall_bytes = 2 * (size_t)s.h_desc->nwc * sizeof(double);
-    if (nwalls < 2 && qw64) RC_CK(cudaMemsetAsync(qw64, 0, wall_bytes, st));
-    if (nwalls < 2 && vw64) RC_CK(cudaMemsetAsync(vw64, 0, wall_bytes, st));
     rc = im.launch_march(s.d_desc, *s.h_desc, s.h_desc->n_tiles, s.d_counter, c->block, st);
     if (rc) return rc;
     rc = im.launch_tally(s.d_desc, s.d_out, 1, im.tally_cells(), st);
