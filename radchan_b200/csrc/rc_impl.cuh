@@ -189,14 +189,15 @@ struct SlotCommon {
     double *d_partial = nullptr;
     size_t partial_cap = 0;
     // the results, one block on the device: q64 | var64 | qw64 | vw64 (double),
-    // Qc | Sc | Wq | Ws (float); pinned staging of the whole block when it is
-    // small (h_all), else of the floats only
+    // Qc | Sc | Wq | Ws (float); pinned staging of the floats, and of the whole
+    // block (stage_block)
     double *d_res = nullptr;
-    unsigned char *h_res = nullptr;
-    bool h_all = false;
+    float *h_res = nullptr;
+    unsigned char *h_stage = nullptr;
+    bool stage_tried = false;
     double *d_q64 = nullptr, *d_var64 = nullptr, *d_qw64 = nullptr, *d_vw64 = nullptr;
     float *d_Qc = nullptr, *d_Sc = nullptr, *d_Wq = nullptr, *d_Ws = nullptr;
-    float *h_Qc = nullptr, *h_Sc = nullptr, *h_Wq = nullptr, *h_Ws = nullptr;
+    float *h_Qc = nullptr, *h_Sc = nullptr;
     unsigned long long *d_counter = nullptr;
     TallyOut *d_out = nullptr, *h_out = nullptr;
     // long-ray priority list (k_prio_tiles): listed tiles, per-tile flag,
@@ -332,6 +333,8 @@ struct Impl : ImplBase {
             dfree(s.d_partial);
             dfree(s.d_res);
             hfree(s.h_res);
+            hfree(s.h_stage);
+            s.stage_tried = false;
             dfree(s.d_counter);
             dfree(s.d_out);
             hfree(s.h_out);
@@ -390,8 +393,22 @@ struct Impl : ImplBase {
     // pageable memory costs about 10 us of waiting, and rc_collect has up to
     // four of them (16^3 grey: 321 -> 255 us a call with the merged set-up
     // kernels).  Above it the extra pass
-    // over host memory would cost more than the waits.
+    // over host memory would cost more than the waits.  A slot's block is
+    // pinned by its first collect that asks for doubles: callers that take
+    // floats or collect on the device do not pay for it.  (Pinned with the
+    // context it made creating one of 64x64x16 cells cost 6.1-6.6 ms, in place
+    // of 4.4-4.8.)
     static constexpr size_t kStageAll = (size_t)2 << 20;
+    static const unsigned char *stage_block(Slot<R> &s, size_t bytes) {
+        if (!s.stage_tried && bytes <= kStageAll) {
+            s.stage_tried = true;
+            if (cudaHostAlloc((void **)&s.h_stage, bytes, cudaHostAllocDefault) != cudaSuccess) {
+                cudaGetLastError();  // without it: the copies go to the caller's arrays
+                s.h_stage = nullptr;
+            }
+        }
+        return s.h_stage;
+    }
 
     // Table coordinates of a level with its halo.
     long long level_cells(int l) const {
@@ -464,13 +481,9 @@ struct Impl : ImplBase {
             s.d_Sc = s.d_Qc + ncf;
             s.d_Wq = s.d_Sc + ncf;
             s.d_Ws = s.d_Wq + nwc;
-            s.h_all = nd * sizeof(double) + nf * sizeof(float) <= kStageAll;
-            RC_CK(cudaHostAlloc((void **)&s.h_res, (s.h_all ? nd * sizeof(double) : 0) + nf * sizeof(float),
-                                cudaHostAllocDefault));
-            s.h_Qc = reinterpret_cast<float *>(s.h_res + (s.h_all ? nd * sizeof(double) : 0));
+            RC_CK(cudaHostAlloc((void **)&s.h_res, nf * sizeof(float), cudaHostAllocDefault));
+            s.h_Qc = s.h_res;
             s.h_Sc = s.h_Qc + ncf;
-            s.h_Wq = s.h_Sc + ncf;
-            s.h_Ws = s.h_Wq + nwc;
             RC_CK(cudaMalloc((void **)&s.d_counter, sizeof(unsigned long long)));
             RC_CK(cudaMalloc((void **)&s.d_out, sizeof(TallyOut)));
             RC_CK(cudaHostAlloc((void **)&s.h_out, sizeof(TallyOut), cudaHostAllocDefault));
@@ -1306,9 +1319,10 @@ struct Impl : ImplBase {
         const size_t ncf = (size_t)p.imax * p.jmax * c->kloc;
         const size_t nwc = (size_t)2 * p.jmax * c->kloc;
         const size_t nd = 2 * ncf + 2 * nwc;
-        const bool all = s.h_all && (q64 || var64 || qw64 || vw64);
+        const size_t nbytes = nd * (sizeof(double) + sizeof(float));
+        const unsigned char *all = q64 || var64 || qw64 || vw64 ? stage_block(s, nbytes) : nullptr;
         if (all) {
-            RC_CK(cudaMemcpyAsync(s.h_res, s.d_res, nd * (sizeof(double) + sizeof(float)), cudaMemcpyDeviceToHost, s.st));
+            RC_CK(cudaMemcpyAsync(s.h_stage, s.d_res, nbytes, cudaMemcpyDeviceToHost, s.st));
         } else {
             if (Q || sigma) RC_CK(cudaMemcpyAsync(s.h_Qc, s.d_Qc, nd * sizeof(float), cudaMemcpyDeviceToHost, s.st));
             if (q64) RC_CK(cudaMemcpyAsync(q64, s.d_q64, ncf * sizeof(double), cudaMemcpyDeviceToHost, s.st));
@@ -1318,19 +1332,19 @@ struct Impl : ImplBase {
         }
         RC_CK(cudaStreamSynchronize(s.st));
         if (all) {
-            const double *h = reinterpret_cast<const double *>(s.h_res);
+            const double *h = reinterpret_cast<const double *>(all);
             if (q64) memcpy(q64, h, ncf * sizeof(double));
             if (var64) memcpy(var64, h + ncf, ncf * sizeof(double));
             if (qw64) memcpy(qw64, h + 2 * ncf, nwc * sizeof(double));
             if (vw64) memcpy(vw64, h + 2 * ncf + nwc, nwc * sizeof(double));
         }
-        if (Q || sigma) scatter(s, Q, sigma);
+        if (Q || sigma) {
+            const float *f = all ? reinterpret_cast<const float *>(all + nd * sizeof(double)) : s.h_Qc;
+            scatter_from(f, f + ncf, f + 2 * ncf, f + 2 * ncf + nwc, Q, sigma);
+        }
         if (const char *bad = status_error(s.h_sc->status)) return set_err(err_, RC_E_RANGE, bad);
         return RC_OK;
     }
-
-    // Fortran layout (0:imax+1, 0:jmax+1, 0:kloc+1) (mc_gpu_noint.cu:975-1005).
-    void scatter(Slot<R> &s, float *Q, float *sigma) { scatter_from(s.h_Qc, s.h_Sc, s.h_Wq, s.h_Ws, Q, sigma); }
 
     // Float results of a batch member from the batch's packed host copy
     // (Q, sigma, wall flux, wall sigma one after the other at `pack`).
@@ -1355,6 +1369,7 @@ struct Impl : ImplBase {
         seg[3] = CopySeg{s.d_Ws, dst + 2 * ncf + nwc, nwc};
     }
 
+    // Fortran layout (0:imax+1, 0:jmax+1, 0:kloc+1) (mc_gpu_noint.cu:975-1005).
     void scatter_from(const float *Qc, const float *Sc, const float *Wq, const float *Ws, float *Q, float *sigma) {
         const rc_params &p = c->p;
         const int im = p.imax, jm = p.jmax, kl = c->kloc;
