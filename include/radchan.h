@@ -286,7 +286,8 @@ int rc_solve_info_get(rc_ctx *ctx, rc_ticket ticket, rc_solve_info *info);
  * 3 or 4; 3 is 72 registers, which also fits seven 128-thread blocks).  None of them changes which bundles are traced. */
 int rc_set_launch(rc_ctx *ctx, int rays_per_thread, int block_threads, int sort_bands, int occupancy);
 int rc_get_launch(rc_ctx *ctx, int *rays_per_thread, int *block_threads, int *sort_bands, int *occupancy);
-/* Long-ray priority of rc_solve_async / rc_solve_device_async.  A bundle
+/* Long-ray priority of rc_solve_async, rc_solve_device_async and the members
+ * of a batch (a captured batch follows a change at its next run).  A bundle
  * whose path is long -- nearly parallel to the x walls, so that it crosses
  * the periodic y/z boundaries again and again, and in a near-transparent
  * band and g point -- takes up to the last level's step budget, and when it

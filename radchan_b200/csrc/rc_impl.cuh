@@ -236,8 +236,8 @@ struct rc_ctx {
     int num_sms = 148;
     bool has_tables = false;
     // changes with every call that changes what a solve's descriptor holds
-    // (tables, particles, launch knobs): a batch captured before such a
-    // change is captured again
+    // (tables, particles, launch knobs) or how it is launched (long-ray
+    // priority): a batch captured before such a change is captured again
     unsigned long long gen = 0;
     // DNS-coupling scratch (rc_dns_source): T1 pencil + four outputs, and a counter
     double *d_dns = nullptr;

@@ -285,6 +285,8 @@ int rc_set_priority(rc_ctx *c, float threshold) {
     if (!c) return set_err(nullptr, RC_E_INVALID, "NULL context");
     if (!(threshold >= 0.f) || threshold > 1e9f)
         return set_err(&c->err, RC_E_INVALID, "threshold must be a path length in [0, 1e9] channel widths");
+    // a captured batch holds the choice of its members' lists
+    if (threshold != c->prio_thr) c->gen++;
     c->prio_thr = threshold;
     return RC_OK;
 }
