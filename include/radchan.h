@@ -359,7 +359,8 @@ int rc_last_error(const rc_ctx *ctx, char *buf, size_t len);
  * so no device fault is involved.  count 0 disarms.  Sites: "field_copy"
  * (a solve's field copy and set-up), "march" and "tally" (their launches),
  * "collect" (result copies), "dns" (the DNS coupling launch), "quantum"
- * (a server march launch). */
+ * (a server march launch), "list" (the memory of a long-ray list: not an
+ * error, the solve goes on without it). */
 int rc_debug_fail_next(const char *site, int count);
 /* Grid faces/centres of level `level` as built by the library
  * (definitions.h:68-136); any pointer may be NULL. */

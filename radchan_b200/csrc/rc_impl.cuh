@@ -206,8 +206,8 @@ struct SlotCommon {
     unsigned *d_prio = nullptr, *d_nprio = nullptr;
     unsigned char *d_tprio = nullptr;
     float *d_kmin = nullptr;
-    long long prio_cap = 0;
-    int kmin_cap = 0;
+    unsigned char *d_list = nullptr;  // the one allocation they are views of
+    size_t list_cap = 0;
     // what the list was built for: the work decomposition and the draws; the
     // list is kept while those stay the same (a later field only changes how
     // well it orders the work, never a result)
@@ -338,12 +338,8 @@ struct Impl : ImplBase {
             dfree(s.d_counter);
             dfree(s.d_out);
             hfree(s.h_out);
-            dfree(s.d_prio);
-            dfree(s.d_tprio);
-            dfree(s.d_nprio);
-            dfree(s.d_kmin);
-            s.prio_cap = 0;
-            s.kmin_cap = 0;
+            dfree(s.d_list);
+            s.list_cap = 0;
             s.prio_ok = false;
             dfree(s.d_levAll);
             s.d_levT.clear();
@@ -960,27 +956,28 @@ struct Impl : ImplBase {
                                    (long long)d.kloc | ((long long)d.kfirst << 32), nt,
                                    (long long)d.nwalls | ((long long)d.wall_id[0] << 8) | ((long long)d.wall_id[1] << 16),
                                    (long long)thr_bits, (long long)sizeof(R)};
-        if (s.prio_ok && s.prio_cap >= nt && memcmp(key, s.prio_key, sizeof(key)) == 0) {
+        if (s.prio_ok && memcmp(key, s.prio_key, sizeof(key)) == 0) {
             use = true;
             return RC_OK;
         }
         s.prio_ok = false;
-        if (s.prio_cap < nt) {
-            dfree(s.d_prio);
-            dfree(s.d_tprio);
-            s.prio_cap = 0;
-            RC_CK(cudaMalloc((void **)&s.d_prio, nt * sizeof(unsigned)));
-            RC_CK(cudaMalloc((void **)&s.d_tprio, nt));
-            s.prio_cap = nt;
-        }
         const int nbq = d.nB * d.nQ;
-        if (s.kmin_cap < nbq) {
-            dfree(s.d_kmin);
-            s.kmin_cap = 0;
-            RC_CK(cudaMalloc((void **)&s.d_kmin, nbq * sizeof(float)));
-            s.kmin_cap = nbq;
+        const size_t bytes = 2 * sizeof(unsigned) + nbq * sizeof(float) + nt * (sizeof(unsigned) + 1);
+        if (s.list_cap < bytes) {
+            dfree(s.d_list);
+            s.list_cap = 0;
+            if (fail_now("list") || cudaMalloc((void **)&s.d_list, bytes) != cudaSuccess) {
+                // the order is all that the list gives: no memory, no list
+                cudaGetLastError();
+                s.d_list = nullptr;
+                return RC_OK;
+            }
+            s.list_cap = bytes;
         }
-        if (!s.d_nprio) RC_CK(cudaMalloc((void **)&s.d_nprio, 2 * sizeof(unsigned)));
+        s.d_nprio = reinterpret_cast<unsigned *>(s.d_list);
+        s.d_kmin = reinterpret_cast<float *>(s.d_nprio + 2);
+        s.d_prio = reinterpret_cast<unsigned *>(s.d_kmin + nbq);
+        s.d_tprio = reinterpret_cast<unsigned char *>(s.d_prio + nt);
         RC_CK(cudaMemsetAsync(s.d_nprio, 0, 2 * sizeof(unsigned), st));
         k_prio_kmin<R><<<(nbq + 255) / 256, 256, 0, st>>>(desc_dev, s.d_kmin);
         RC_CK(cudaGetLastError());

@@ -342,7 +342,7 @@ int rc_last_error(const rc_ctx *c, char *buf, size_t len) {
 }
 
 int rc_debug_fail_next(const char *site, int count) {
-    static const char *const sites[] = {"field_copy", "march", "tally", "collect", "dns", "quantum"};
+    static const char *const sites[] = {"field_copy", "march", "tally", "collect", "dns", "quantum", "list"};
     if (!site || count < 0) return set_err(nullptr, RC_E_INVALID, "NULL site or negative count");
     bool known = false;
     for (const char *s : sites) known = known || strcmp(s, site) == 0;

@@ -1,7 +1,7 @@
 """A batch that has been captured follows a later rc_set_priority of its
 members: the next run builds the launches again (seen by the failure armed at
 the march's launch, which a plain replay never meets) and the results keep
-every bit."""
+every bit.  A list that finds no memory is left out: it is an order only."""
 import numpy as np
 import pytest
 
@@ -12,8 +12,8 @@ from radchan_b200 import workloads as W
 pytestmark = pytest.mark.gpu
 
 
-def _arm(n):
-    L.check(L.lib().rc_debug_fail_next(b"march", n))
+def _arm(n, site=b"march"):
+    L.check(L.lib().rc_debug_fail_next(site, n))
 
 
 def test_captured_batch_follows_set_priority():
@@ -52,3 +52,30 @@ def test_captured_batch_follows_set_priority():
     b.close()
     for s in ss:
         s.close()
+
+
+def test_no_memory_for_the_list_is_no_failure():
+    p = W.channel_params(12, 10, 8, grey=True, photmax=20, nVar=2)
+    T = W.channel_field(p, seed=3)
+    s = api.Solver(p)
+    ref = s.solve(T)
+    s.close()
+    try:
+        s = api.Solver(p)
+        _arm(1, b"list")
+        for _ in range(2):  # without the list, then with it
+            np.testing.assert_array_equal(s.solve(T).q64, ref.q64)
+        for graph in (False, True):
+            b = api.Batch(use_graph=graph)
+            x = api.Solver(p)
+            b.add(x, T)
+            _arm(1, b"list")
+            for _ in range(2):
+                b.run()
+                b.wait()
+                np.testing.assert_array_equal(b.collect(0).q64, ref.q64)
+            b.close()
+            x.close()
+        s.close()
+    finally:
+        _arm(0, b"list")
