@@ -469,67 +469,62 @@ int batch_join(rc_batch *b, int ns) {
     return RC_OK;
 }
 
-// First part of a batch on b->st: per member field copy + set-up.
+// Host half of a run: descriptors, tally outputs and copy segments of every
+// member, in pinned memory that the device half copies from.  Written once per
+// run or capture, with nothing of the batch in flight.
 template <typename R>
-int batch_enqueue_setup(rc_batch *b) {
-    std::string *err_ = &b->err;
-    const size_t n = b->m.size();
-    int rc = batch_reserve<R>(b, n);
-    if (rc) return rc;
+int batch_fill(rc_batch *b) {
     DSolve<R> *hs = static_cast<DSolve<R> *>(b->h_solves);
-    // host halves: descriptors, tally outputs of every member
-    long long maxf = 1;
+    const size_t n = b->m.size();
     for (size_t i = 0; i < n; ++i) {
         rc_ctx *c = b->m[i].ctx;
         Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
         Slot<R> &s = *static_cast<Slot<R> *>(b->m[i].slot);
-        rc = im.prepare_host(s, b->m[i].zstart, c->rpt);
-        if (rc) return set_err(err_, rc, c->err);
+        const int rc = im.prepare_host(s, b->m[i].zstart, c->rpt);
+        if (rc) return set_err(&b->err, rc, c->err);
         hs[i] = *s.h_desc;
         b->h_outs[i] = *s.h_out;
         b->h_segs[i] = CopySeg{s.h_T, s.d_T, (long long)im.field_floats()};
-        maxf = std::max(maxf, b->h_segs[i].n);
+        im.pack_segments(s, b->d_pack + b->pack_off[i], b->h_segs + n + 4 * i);
     }
+    return RC_OK;
+}
+
+// First part of a batch on b->st: per member field copy and set-up, and
+// (lists) the long-ray priority lists that are not up to date -- never
+// captured, as a list is kept (see enqueue_prio).
+template <typename R>
+int batch_enqueue_setup(rc_batch *b, bool lists) {
+    std::string *err_ = &b->err;
+    const size_t n = b->m.size();
+    DSolve<R> *hs = static_cast<DSolve<R> *>(b->h_solves);
+    long long maxf = 1;
+    for (size_t i = 0; i < n; ++i) maxf = std::max(maxf, b->h_segs[i].n);
     // one copy each of the descriptors and tally outputs; every member's
     // field in one launch that reads the pinned staging directly
     RC_CK(cudaMemcpyAsync(b->d_solves, hs, n * sizeof(DSolve<R>), cudaMemcpyHostToDevice, b->st));
     RC_CK(cudaMemcpyAsync(b->d_outs, b->h_outs, n * sizeof(TallyOut), cudaMemcpyHostToDevice, b->st));
-    RC_CK(cudaMemcpyAsync(b->d_segs, b->h_segs, n * sizeof(CopySeg), cudaMemcpyHostToDevice, b->st));
+    RC_CK(cudaMemcpyAsync(b->d_segs, b->h_segs, 5 * n * sizeof(CopySeg), cudaMemcpyHostToDevice, b->st));
     k_copy_segs<<<dim3((unsigned)std::min<long long>((maxf + 255) / 256, 64), (unsigned)n), 256, 0, b->st>>>(b->d_segs);
     RC_CK(cudaGetLastError());
-    // every member's set-up kernels, round-robin over the side streams:
-    // independent chains that run side by side, patching the batch's
+    // every member's set-up kernels and list, round-robin over the side
+    // streams: independent chains that run side by side, patching the batch's
     // descriptors in place
     const int ns = (int)std::min<size_t>(n, (size_t)rc_batch::kSideStreams);
-    rc = batch_fork(b, ns);
+    int rc = batch_fork(b, ns);
     if (rc) return rc;
     int rc_members = RC_OK;
     for (size_t i = 0; i < n && !rc_members; ++i) {
         rc_ctx *c = b->m[i].ctx;
         Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
         Slot<R> &s = *static_cast<Slot<R> *>(b->m[i].slot);
-        rc = im.prepare_device(s, nullptr, true, static_cast<DSolve<R> *>(b->d_solves) + i, b->side[i % ns]);
+        DSolve<R> *d = static_cast<DSolve<R> *>(b->d_solves) + i;
+        rc = im.prepare_device(s, nullptr, true, d, b->side[i % ns]);
+        if (!rc && lists) rc = im.enqueue_prio(s, b->side[i % ns], b->m[i].prio, d);
         if (rc) rc_members = set_err(err_, rc, c->err);
     }
     rc = batch_join(b, ns);
     return rc ? rc : rc_members;
-}
-
-// Long-ray priority lists of the members whose list is not up to date, after
-// their set-up on b->st (never captured: a list is kept, see enqueue_prio).
-template <typename R>
-int batch_enqueue_prio(rc_batch *b) {
-    std::string *err_ = &b->err;
-    for (size_t i = 0; i < b->m.size(); ++i) {
-        rc_ctx *c = b->m[i].ctx;
-        Impl<R> &im = *static_cast<Impl<R> *>(c->impl);
-        bool use = false;
-        int rc = im.enqueue_prio(*static_cast<Slot<R> *>(b->m[i].slot), b->st, use,
-                                 static_cast<const DSolve<R> *>(b->d_solves) + i);
-        if (rc) return set_err(err_, rc, c->err);
-        b->m[i].prio = use;
-    }
-    return RC_OK;
 }
 
 // The whole batch on b->st: set-up, every member's march, one tally launch,
@@ -548,8 +543,7 @@ int batch_enqueue(rc_batch *b, bool capturing) {
     };
     const size_t n = b->m.size();
     const int ns = (int)std::min<size_t>(n, (size_t)rc_batch::kSideStreams);
-    int rc = batch_enqueue_setup<R>(b);
-    if (!rc && !capturing) rc = batch_enqueue_prio<R>(b);
+    int rc = batch_enqueue_setup<R>(b, !capturing);
     if (rc) return rc;
     RC_CK(mark(b->e_setup));
     rc = batch_fork(b, ns);
@@ -573,16 +567,10 @@ int batch_enqueue(rc_batch *b, bool capturing) {
     if (rc) return set_err(err_, rc, b->m[0].ctx->err);
     // float results of every member into one buffer, one copy to the host
     long long maxn = 1;
-    CopySeg *rs = b->h_segs + n;
-    for (size_t i = 0; i < n; ++i) {
-        Impl<R> &im = *static_cast<Impl<R> *>(b->m[i].ctx->impl);
-        im.pack_segments(*static_cast<Slot<R> *>(b->m[i].slot), b->d_pack + b->pack_off[i], rs + 4 * i);
-        for (int q = 0; q < 4; ++q) maxn = std::max(maxn, rs[4 * i + q].n);
-    }
+    for (size_t q = n; q < 5 * n; ++q) maxn = std::max(maxn, b->h_segs[q].n);
     size_t floats = 0;
     for (size_t i = 0; i < n; ++i)
         floats += static_cast<Impl<R> *>(b->m[i].ctx->impl)->packed_floats();
-    RC_CK(cudaMemcpyAsync(b->d_segs + n, rs, 4 * n * sizeof(CopySeg), cudaMemcpyHostToDevice, b->st));
     {
         const int gx = (int)std::min<long long>((maxn + 255) / 256, 64);
         k_copy_segs<<<dim3(gx, (unsigned)(4 * n)), 256, 0, b->st>>>(b->d_segs + n);
@@ -708,15 +696,17 @@ int rc_batch_run(rc_batch *b) {
     if (!b->built || !b->use_graph) {
         rc = b->dbl ? batch_reserve_members<double>(b) : batch_reserve_members<float>(b);
         if (rc) return rc;
-    }
-    if (!b->use_graph) {
+        rc = b->dbl ? batch_fill<double>(b) : batch_fill<float>(b);
+        if (rc) return rc;
         RC_CK(cudaEventRecord(b->e0, b->st));
         rc = b->dbl ? batch_enqueue<double>(b, false) : batch_enqueue<float>(b, false);
         if (rc) return rc;
         RC_CK(cudaEventRecord(b->e1, b->st));
-        return RC_OK;
-    }
-    if (!b->built) {
+        if (!b->use_graph) return RC_OK;
+        // the run is on its way; while it works, the same sequence without
+        // the lists (which it builds) is captured for the runs to come
+        // (the members' set-up once more before a captured first run, to build
+        // the lists, made the first run of 96 solves of 8^3 take 9.6 ms, this way 8.5)
         if (b->exec) {
             cudaGraphExecDestroy(b->exec);
             b->exec = nullptr;
@@ -725,13 +715,6 @@ int rc_batch_run(rc_batch *b) {
             cudaGraphDestroy(b->graph);
             b->graph = nullptr;
         }
-        // the priority lists need the members' set-up, which runs once more,
-        // outside the graph, when one has to be built
-        rc = b->dbl ? batch_enqueue_setup<double>(b) : batch_enqueue_setup<float>(b);
-        if (!rc) rc = b->dbl ? batch_enqueue_prio<double>(b) : batch_enqueue_prio<float>(b);
-        if (rc) return rc;
-        // the capture rewrites the pinned descriptors that this set-up reads
-        RC_CK(cudaStreamSynchronize(b->st));
         RC_CK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
         rc = b->dbl ? batch_enqueue<double>(b, true) : batch_enqueue<float>(b, true);
         cudaGraph_t g = nullptr;
@@ -744,6 +727,7 @@ int rc_batch_run(rc_batch *b) {
         b->graph = g;
         RC_CK(cudaGraphInstantiate(&b->exec, b->graph, 0));
         b->built = true;
+        return RC_OK;
     }
     RC_CK(cudaEventRecord(b->e0, b->st));
     RC_CK(cudaGraphLaunch(b->exec, b->st));

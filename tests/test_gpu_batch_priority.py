@@ -55,7 +55,8 @@ def test_captured_batch_follows_set_priority():
 
 
 def test_no_memory_for_the_list_is_no_failure():
-    p = W.channel_params(12, 10, 8, grey=True, photmax=20, nVar=2)
+    # more tiles than the march has warps: below that there is no list
+    p = W.channel_params(32, 24, 20, grey=True, photmax=40, nVar=2)
     T = W.channel_field(p, seed=3)
     s = api.Solver(p)
     ref = s.solve(T)
@@ -79,3 +80,29 @@ def test_no_memory_for_the_list_is_no_failure():
         s.close()
     finally:
         _arm(0, b"list")
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_first_run_equals_later_runs(graph):
+    """The first run of a captured batch goes out before its capture; more
+    members than side streams, one of them without a list."""
+    ps = [W.channel_params(6 + i % 5, 5, 4 + i % 3, grey=True, photmax=6 + i, nVar=2, seed=i) for i in range(19)]
+    ss = [api.Solver(p) for p in ps]
+    T = [W.channel_field(p, seed=9) for p in ps]
+    ss[3].set_priority(0.0)
+    ref = [s.solve(t) for s, t in zip(ss, T)]
+    b = api.Batch(use_graph=graph)
+    for s, t in zip(ss, T):
+        b.add(s, t)
+    for _ in range(3):
+        b.run()
+        assert b.wait() > 0
+        assert all(ms >= 0 for ms in b.phases())
+        for i, r in enumerate(ref):
+            Q, S = (np.zeros(api.result_shape(ps[i]), np.float32) for _ in range(2))
+            b.collect_into(i, Q, S)
+            np.testing.assert_array_equal(Q, r.Q)
+            np.testing.assert_array_equal(b.collect(i).var64, r.var64)
+    b.close()
+    for s in ss:
+        s.close()
