@@ -297,7 +297,10 @@ int rc_get_launch(rc_ctx *ctx, int *rays_per_thread, int *block_threads, int *so
  * ln(1/tol) / k_min) (d_x the distance to the x wall it heads for, k_min the
  * smallest k of its band and g point over the table rows the field spans)
  * and lists the tiles holding a bundle whose estimate exceeds `threshold`
- * channel widths Lx; the march claims those tiles first.  Default
+ * channel widths Lx; the march claims those tiles first, and the ones whose
+ * estimate exceeds 16 thresholds before the others.  While these last are no
+ * more than the launch's warps, a warp that has claimed one takes nothing else
+ * until its rays have finished, so that they are stepped more often.  Default
  * RC_PRIORITY_DEFAULT; 0 turns it off.  It changes the order of the work,
  * never a result.  Each solve slot builds the list on its first solve and
  * reuses it while the draws and the work decomposition stay the same (seed,

@@ -81,7 +81,12 @@ struct MarchParams {
 // L > kSoloPath * thr * Lx.  Such a ray decides when a short launch ends: a
 // warp that has claimed its tile claims no other before its rays have
 // finished, so the ray is not held up by the emission and feeding of others
-// (its warp then steps it 2-3 times as often).  The draws are the emission's own (Philox
+// (its warp then steps it 2-3 times as often).  That holds as long as there is
+// a warp for every such tile; with more of them (a near-transparent gas, a low
+// threshold) warps that step one ray each would be the rule, and the tiles are
+// only claimed early (grey 32^3, k 0.01 1/m: 19.3 ms with a warp held for every
+// one, 10.6 so; k 0.001: 51 and 37 ms; narrow-band cases with a handful of such
+// tiles, 20-30% faster by the hold, are the same).  The draws are the emission's own (Philox
 // counter of the bundle, select_band_g), so the estimate sees the same
 // direction, band and g point the march will trace.  Only the order in
 // which tiles are claimed changes, never a result.
@@ -259,8 +264,9 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
                     }
                     if (!np) break;
                     if (tile < nprio) {
-                        hold = tile < nsolo;
-                        tile = __ldg(a.prio_tiles + (hold ? tile : (unsigned long long)a.total_tiles - 1 - (tile - nsolo)));
+                        const bool solo = tile < nsolo;
+                        hold = solo && nsolo <= gridDim.x * nwarps;
+                        tile = __ldg(a.prio_tiles + (solo ? tile : (unsigned long long)a.total_tiles - 1 - (tile - nsolo)));
                         break;
                     }
                     if (!__ldg(a.tile_prio + (tile - nprio))) {
