@@ -189,12 +189,9 @@ struct SlotCommon {
     double *d_partial = nullptr;
     size_t partial_cap = 0;
     // the results, one block on the device: q64 | var64 | qw64 | vw64 (double),
-    // Qc | Sc | Wq | Ws (float); pinned staging of the floats, and of the whole
-    // block (stage_block)
+    // Qc | Sc | Wq | Ws (float); pinned staging of the floats from h_Qc on
     double *d_res = nullptr;
-    float *h_res = nullptr;
-    unsigned char *h_stage = nullptr;
-    bool stage_tried = false;
+    unsigned char *h_pin = nullptr;  // the slot's pinned memory (Impl::pin): h_T, h_Qc, h_sc, h_out, h_desc
     double *d_q64 = nullptr, *d_var64 = nullptr, *d_qw64 = nullptr, *d_vw64 = nullptr;
     float *d_Qc = nullptr, *d_Sc = nullptr, *d_Wq = nullptr, *d_Ws = nullptr;
     float *h_Qc = nullptr, *h_Sc = nullptr;
@@ -327,17 +324,12 @@ struct Impl : ImplBase {
         for (auto &s : slots) {
             if (s.st) cudaStreamSynchronize(s.st);
             dfree(s.d_T);
-            hfree(s.h_T);
             dfree(s.d_sc);
-            hfree(s.h_sc);
             dfree(s.d_partial);
             dfree(s.d_res);
-            hfree(s.h_res);
-            hfree(s.h_stage);
-            s.stage_tried = false;
+            hfree(s.h_pin);
             dfree(s.d_counter);
             dfree(s.d_out);
-            hfree(s.h_out);
             dfree(s.d_list);
             s.list_cap = 0;
             s.prio_ok = false;
@@ -357,7 +349,6 @@ struct Impl : ImplBase {
             dfree(s.d_Tnb_grey);
             dfree(s.d_Ibt_grey);
             dfree(s.d_desc);
-            hfree(s.h_desc);
             if (s.e0) cudaEventDestroy(s.e0);
             if (s.e1) cudaEventDestroy(s.e1);
             if (s.e_march0) cudaEventDestroy(s.e_march0);
@@ -366,6 +357,9 @@ struct Impl : ImplBase {
             if (s.st) cudaStreamDestroy(s.st);
         }
         slots.clear();
+        if (stage_own) hfree(h_stage);
+        h_stage = nullptr;
+        stage_own = stage_tried = false;
         dfree(d_faces);
         d_xu.clear();
         d_yu.clear();
@@ -389,21 +383,60 @@ struct Impl : ImplBase {
     // pageable memory costs about 10 us of waiting, and rc_collect has up to
     // four of them (16^3 grey: 321 -> 255 us a call with the merged set-up
     // kernels).  Above it the extra pass
-    // over host memory would cost more than the waits.  A slot's block is
-    // pinned by its first collect that asks for doubles: callers that take
-    // floats or collect on the device do not pay for it.  (Pinned with the
-    // context it made creating one of 64x64x16 cells cost 6.1-6.6 ms, in place
-    // of 4.4-4.8.)
-    static constexpr size_t kStageAll = (size_t)2 << 20;
-    static const unsigned char *stage_block(Slot<R> &s, size_t bytes) {
-        if (!s.stage_tried && bytes <= kStageAll) {
-            s.stage_tried = true;
-            if (cudaHostAlloc((void **)&s.h_stage, bytes, cudaHostAllocDefault) != cudaSuccess) {
-                cudaGetLastError();  // without it: the copies go to the caller's arrays
-                s.h_stage = nullptr;
+    // over host memory would cost more than the waits.  The
+    // block is pinned with the context's first slot while both together stay
+    // within kPinRoom, and else by the first collect that asks for doubles;
+    // the second slot's memory is pinned when a second solve is first in
+    // flight.  Pinning costs about 1 ms a megabyte, so a program that solves
+    // one field at a time, takes floats or collects on the device does not
+    // pay for what it does not use.  (Create and first solve, ms, every slot
+    // with a block from the start / now: 64x64x16
+    // cells 8.5 and 1.8 / 4.5 and 1.4 collected on the device; grey 32^3 6.3
+    // and 0.8 / 5.7 and 0.8; 64^3 11.1 and 6.3 / 8.5 and 6.3.)
+    static constexpr size_t kStageAll = (size_t)2 << 20, kPinRoom = (size_t)2 << 20;
+    unsigned char *h_stage = nullptr;
+    bool stage_tried = false, stage_own = false;
+    int pin_rc = RC_OK;  // of the last free_slot
+    std::mutex stage_mu;  // the block serves both slots, one copy at a time
+    size_t result_bytes() const {
+        const size_t nc = (size_t)c->p.imax * c->p.jmax * c->kloc + (size_t)2 * c->p.jmax * c->kloc;
+        return 2 * nc * (sizeof(double) + sizeof(float));
+    }
+    const unsigned char *stage_block() {
+        if (!stage_tried) {
+            stage_tried = true;
+            if (!h_stage && result_bytes() <= kStageAll) {
+                stage_own = cudaHostAlloc((void **)&h_stage, result_bytes(), cudaHostAllocDefault) == cudaSuccess;
+                if (!stage_own) {
+                    cudaGetLastError();  // without it: the copies go to the caller's arrays
+                    h_stage = nullptr;
+                }
             }
         }
-        return s.h_stage;
+        return h_stage;
+    }
+    // Pinned memory of a slot, and of the block when it goes with it.
+    int pin(Slot<R> &s, bool with_block) {
+        std::string *err_ = &c->err;
+        auto up = [](size_t n) { return (n + 255) & ~(size_t)255; };
+        const size_t floats = result_bytes() / (sizeof(double) + sizeof(float));
+        const size_t bT = up(field_floats() * sizeof(float)), bF = up(floats * sizeof(float)), bS = up(sizeof(DScalars)),
+                     bO = up(sizeof(TallyOut)), bD = up(sizeof(DSolve<R>)), slot = bT + bF + bS + bO + bD;
+        with_block = with_block && slot + result_bytes() <= kPinRoom;
+        RC_CK(cudaHostAlloc((void **)&s.h_pin, slot + (with_block ? result_bytes() : 0), cudaHostAllocDefault));
+        unsigned char *q = s.h_pin;
+        auto take = [&](auto *&dst, size_t n) {
+            dst = reinterpret_cast<std::remove_reference_t<decltype(dst)>>(q);
+            q += n;
+        };
+        take(s.h_T, bT);
+        take(s.h_Qc, bF);
+        take(s.h_sc, bS);
+        take(s.h_out, bO);
+        take(s.h_desc, bD);
+        s.h_Sc = s.h_Qc + (size_t)c->p.imax * c->p.jmax * c->kloc;
+        if (with_block) h_stage = q;
+        return RC_OK;
     }
 
     // Table coordinates of a level with its halo.
@@ -454,6 +487,8 @@ struct Impl : ImplBase {
         const size_t nfield = (size_t)(p.imax + 2) * (p.jmax + 2) * (p.kmax + 2);
         const size_t ncf = (size_t)p.imax * p.jmax * c->kloc;
         const size_t nwc = (size_t)2 * p.jmax * c->kloc;
+        rc = pin(slots[0], true);
+        if (rc) return rc;
         for (auto &s : slots) {
             RC_CK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
             RC_CK(cudaEventCreate(&s.e0));
@@ -461,9 +496,7 @@ struct Impl : ImplBase {
             RC_CK(cudaEventCreate(&s.e_march0));
             RC_CK(cudaEventCreate(&s.e_march1));
             RC_CK(cudaMalloc((void **)&s.d_T, nfield * sizeof(float)));
-            RC_CK(cudaHostAlloc((void **)&s.h_T, nfield * sizeof(float), cudaHostAllocDefault));
             RC_CK(cudaMalloc((void **)&s.d_sc, sizeof(DScalars)));
-            RC_CK(cudaHostAlloc((void **)&s.h_sc, sizeof(DScalars), cudaHostAllocDefault));
             const size_t nd = 2 * ncf + 2 * nwc, nf = nd;  // doubles, floats of the results
             RC_CK(cudaMalloc((void **)&s.d_res, nd * sizeof(double) + nf * sizeof(float)));
             // (nothing is cleared here: a memset on the default stream is not
@@ -477,14 +510,9 @@ struct Impl : ImplBase {
             s.d_Sc = s.d_Qc + ncf;
             s.d_Wq = s.d_Sc + ncf;
             s.d_Ws = s.d_Wq + nwc;
-            RC_CK(cudaHostAlloc((void **)&s.h_res, nf * sizeof(float), cudaHostAllocDefault));
-            s.h_Qc = s.h_res;
-            s.h_Sc = s.h_Qc + ncf;
             RC_CK(cudaMalloc((void **)&s.d_counter, sizeof(unsigned long long)));
             RC_CK(cudaMalloc((void **)&s.d_out, sizeof(TallyOut)));
-            RC_CK(cudaHostAlloc((void **)&s.h_out, sizeof(TallyOut), cudaHostAllocDefault));
             RC_CK(cudaMalloc((void **)&s.d_desc, sizeof(DSolve<R>)));
-            RC_CK(cudaHostAlloc((void **)&s.h_desc, sizeof(DSolve<R>), cudaHostAllocDefault));
             // multigrid pyramid and wall emission arrays
             s.d_levT.assign(nl, nullptr);
             {
@@ -1046,9 +1074,12 @@ struct Impl : ImplBase {
 
     Slot<R> *free_slot() {
         for (auto &s : slots)
-            if (s.state == 0) return &s;
+            if (s.state == 0) return s.h_pin || (pin_rc = pin(s, false)) == RC_OK ? &s : nullptr;
+        pin_rc = RC_OK;
         return nullptr;
     }
+    // Why free_slot gave none.
+    int no_slot(const char *busy) { return pin_rc ? pin_rc : set_err(&c->err, RC_E_BUSY, busy); }
 
     int check_solve_args(const float *T, int zstart) {
         std::string *err_ = &c->err;
@@ -1147,7 +1178,7 @@ struct Impl : ImplBase {
         int rc = check_solve_args(T, zstart);
         if (rc) return rc;
         Slot<R> *sp = free_slot();
-        if (!sp) return set_err(err_, RC_E_BUSY, "all solve slots in use: collect a ticket first");
+        if (!sp) return no_slot("all solve slots in use: collect a ticket first");
         Slot<R> &s = *sp;
         const int rpt = c->rpt;
         if (!device_ptr) {
@@ -1214,7 +1245,7 @@ struct Impl : ImplBase {
         int rc = check_solve_args(T, zstart);
         if (rc) return rc;
         Slot<R> *sp = free_slot();
-        if (!sp) return set_err(err_, RC_E_BUSY, "all solve slots in use");
+        if (!sp) return no_slot("all solve slots in use");
         Slot<R> &s = *sp;
         const int saved_photmax = c->p.photmax, saved_sort = c->sort;
         // the pilot is raised until its launch has 10^8 bundles or more
@@ -1334,10 +1365,14 @@ struct Impl : ImplBase {
         const size_t ncf = (size_t)p.imax * p.jmax * c->kloc;
         const size_t nwc = (size_t)2 * p.jmax * c->kloc;
         const size_t nd = 2 * ncf + 2 * nwc;
-        const size_t nbytes = nd * (sizeof(double) + sizeof(float));
-        const unsigned char *all = q64 || var64 || qw64 || vw64 ? stage_block(s, nbytes) : nullptr;
+        std::unique_lock<std::mutex> lk(stage_mu, std::defer_lock);
+        const unsigned char *all = nullptr;
+        if (q64 || var64 || qw64 || vw64) {
+            lk.lock();
+            all = stage_block();
+        }
         if (all) {
-            RC_CK(cudaMemcpyAsync(s.h_stage, s.d_res, nbytes, cudaMemcpyDeviceToHost, s.st));
+            RC_CK(cudaMemcpyAsync(h_stage, s.d_res, result_bytes(), cudaMemcpyDeviceToHost, s.st));
         } else {
             if (Q || sigma) RC_CK(cudaMemcpyAsync(s.h_Qc, s.d_Qc, nd * sizeof(float), cudaMemcpyDeviceToHost, s.st));
             if (q64) RC_CK(cudaMemcpyAsync(q64, s.d_q64, ncf * sizeof(double), cudaMemcpyDeviceToHost, s.st));

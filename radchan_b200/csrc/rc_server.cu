@@ -516,8 +516,11 @@ void admit(rc_server *sv) {
         if (!rc) {
             Impl<float> &im = *static_cast<Impl<float> *>(r->ctx->impl);
             r->slot = im.free_slot();
-            r->slot->state = 3;
-            rc = im.stage_host_field(*r->slot, r->T.data());
+            rc = r->slot ? RC_OK : im.no_slot("no free slot in context");
+            if (!rc) {
+                r->slot->state = 3;
+                rc = im.stage_host_field(*r->slot, r->T.data());
+            }
             if (rc) g_err = r->ctx->err;
         }
         std::lock_guard<std::mutex> lk(sv->mu);

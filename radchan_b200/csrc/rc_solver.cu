@@ -654,7 +654,7 @@ int rc_batch_add(rc_batch *b, rc_ctx *c, const float *T_host, int zstart) {
         int r = im.check_solve_args(T_host, zstart);
         if (r) return r;
         auto *s = im.free_slot();
-        if (!s) return set_err(&c->err, RC_E_BUSY, "no free slot in context");
+        if (!s) return im.no_slot("no free slot in context");
         r = im.stage_host_field(*s, T_host);
         if (r) return r;
         s->state = 3;  // reserved by the batch
@@ -875,7 +875,7 @@ int solve_noalloc_t(rc_ctx *c, const float *T_dev, int zstart, double *q64, doub
     rc = noalloc_scratch(c->device, &scratch, err_);
     if (rc) return rc;
     Slot<R> *sp = im.free_slot();
-    if (!sp) return set_err(err_, RC_E_BUSY, "all solve slots in use: collect a ticket first");
+    if (!sp) return im.no_slot("all solve slots in use: collect a ticket first");
     Slot<R> &s = *sp;
     cudaStream_t st = s.st;
     const size_t nfield = (size_t)(p.imax + 2) * (p.jmax + 2) * (p.kmax + 2);
