@@ -203,8 +203,9 @@ struct SlotCommon {
     unsigned *d_prio = nullptr, *d_nprio = nullptr;
     unsigned char *d_tprio = nullptr;
     float *d_kmin = nullptr;
-    unsigned char *d_list = nullptr;  // the one allocation they are views of
+    unsigned char *d_list = nullptr;  // all of them but d_prio
     size_t list_cap = 0;
+    long long prio_cap = 0;
     // what the list was built for: the work decomposition and the draws; the
     // list is kept while those stay the same (a later field only changes how
     // well it orders the work, never a result)
@@ -331,7 +332,9 @@ struct Impl : ImplBase {
             dfree(s.d_counter);
             dfree(s.d_out);
             dfree(s.d_list);
+            dfree(s.d_prio);
             s.list_cap = 0;
+            s.prio_cap = 0;
             s.prio_ok = false;
             dfree(s.d_levAll);
             s.d_levT.clear();
@@ -997,22 +1000,28 @@ struct Impl : ImplBase {
         }
         s.prio_ok = false;
         const int nbq = d.nB * d.nQ;
-        const size_t bytes = 2 * sizeof(unsigned) + nbq * sizeof(float) + nt * (sizeof(unsigned) + 1);
-        if (s.list_cap < bytes) {
+        // (two allocations: the numbers of 2^18 tiles are 1 MB to the byte, and
+        // in one block with the rest they cost a first solve 0.4 ms more)
+        const size_t bytes = 2 * sizeof(unsigned) + nbq * sizeof(float) + nt;
+        if (s.list_cap < bytes || s.prio_cap < nt) {
             dfree(s.d_list);
+            dfree(s.d_prio);
             s.list_cap = 0;
-            if (fail_now("list") || cudaMalloc((void **)&s.d_list, bytes) != cudaSuccess) {
+            s.prio_cap = 0;
+            if (fail_now("list") || cudaMalloc((void **)&s.d_prio, nt * sizeof(unsigned)) != cudaSuccess ||
+                cudaMalloc((void **)&s.d_list, bytes) != cudaSuccess) {
                 // the order is all that the list gives: no memory, no list
                 cudaGetLastError();
                 s.d_list = nullptr;
+                dfree(s.d_prio);
                 return RC_OK;
             }
             s.list_cap = bytes;
+            s.prio_cap = nt;
         }
         s.d_nprio = reinterpret_cast<unsigned *>(s.d_list);
         s.d_kmin = reinterpret_cast<float *>(s.d_nprio + 2);
-        s.d_prio = reinterpret_cast<unsigned *>(s.d_kmin + nbq);
-        s.d_tprio = reinterpret_cast<unsigned char *>(s.d_prio + nt);
+        s.d_tprio = reinterpret_cast<unsigned char *>(s.d_kmin + nbq);
         RC_CK(cudaMemsetAsync(s.d_nprio, 0, 2 * sizeof(unsigned), st));
         k_prio_kmin<R><<<(nbq + 255) / 256, 256, 0, st>>>(desc_dev, s.d_kmin);
         RC_CK(cudaGetLastError());
