@@ -55,8 +55,6 @@ struct DLevel {
     int rx, ry, rz;           // ratio to the next (coarser) level
     unsigned mrx, mry, mrz;   // floor(2^32 / r) + 1 (0 for r = 1): (n + r - 1) / r as a multiply-high
     const R *xu, *yu, *zu;    // faces (views into DSolve::faces)
-    const uint16_t *P;        // table coordinate of every cell and its halo (see cell_index);
-                              // a view into DSolve::Pall
     const uint16_t *Pw[6];    // wall emission temperature coordinates (or null)
 };
 
@@ -89,7 +87,7 @@ struct DSolve {
     // lvb = (km, maxs, bits of dy, bits of dz): face j of y lies at j dy
     int4 lva[RC_MAX_LEVELS], lvb[RC_MAX_LEVELS];
     const R *faces;           // every level's xu | yu | zu, one after the other
-    const uint16_t *Pall;     // every level's table coordinates, one after the other
+    const uint16_t *Pall;     // every level's table coordinates with their halos (cell_index), one after the other
     DLevel<R> lev[RC_MAX_LEVELS];
     int nlev;
     int imax, jmax, kmax, kloc, kfirst;
@@ -98,15 +96,12 @@ struct DSolve {
     int nVar, photmax, rpt, nchunk, gsize, nparts;
     int sort;  // 1: emitted bundles enter the ring in ascending k (band-sorted order)
     int nwalls, wall_id[2];
-    int pad;
     R Lx, Ly, Lz;
     R toll, tollS;
     // run-time values (copied from DScalars by the kernels)
     R Ibmax_f, Ibmax_w0, Ibmax_w1;
-    int Pm, row;
+    int row;
     const R *xc, *yc, *zc;    // level-0 cell centres incl. ghosts
-    const R *kt;              // [nB][nQ][nT]
-    const R *Ibt;             // [nB][nT]
     const R *probg;           // [nT][nB][nQ]
     const R *cdf_f;           // [nB] fluid band CDF at the selected row
     const R *cdf_s;           // [nB] wall band CDF at the selected row
@@ -124,7 +119,6 @@ struct DSolve {
     const R *pth;             // [nA] scattering angles in turns (theta / 2 pi)
     const uint16_t *pguide;   // [nB][kPhaseGuide+1] phase-CDF search brackets (phase_index)
     int nA;
-    int pad3;
     DScalars *sc;
     double *partial;
     long long n_fluid_items, n_items, n_tiles;

@@ -795,7 +795,6 @@ struct Impl : ImplBase {
             L.xu = d_xu[l];
             L.yu = d_yu[l];
             L.zu = d_zu[l];
-            L.P = s.d_levT[l];
             int dy, dz;
             memcpy(&dy, &c->grid[l].dy, 4);
             memcpy(&dz, &c->grid[l].dz, 4);
@@ -833,8 +832,6 @@ struct Impl : ImplBase {
         d.xc = d_xc;
         d.yc = d_yc;
         d.zc = d_zc;
-        d.kt = d_kt;
-        d.Ibt = p.grey ? s.d_Ibt_grey : d_Ibt;
         d.probg = d_probg;
         d.cdf_f = s.d_cdf_f;
         d.cdf_s = s.d_cdf_s;

@@ -99,7 +99,6 @@ __global__ void k_setup1(DScalars *sc, DSolve<R> *d, R *Tnb, const R *kP, int nT
     sc->T0 = (double)T0;
     sc->inv_dT = (double)inv_dT;
     sc->Pm = table_coord(Tmax, T0, inv_dT, nT);
-    d->Pm = sc->Pm;
     d->row = row;
     d->Ibmax_f = (R)sc->Ibmax_f;
     d->Ibmax_w0 = (R)sc->Ibmax_w[0];
