@@ -169,8 +169,9 @@ size_t context_bytes(const rc_params &p, int photmax) {
     const double ncf = (double)p.imax * p.jmax * kl, nwc = 2.0 * p.jmax * kl;
     double slot = nfield * 4 + ncf * 24 + nwc * 24 + 2.0 * p.jmax * p.kmax * 2;
     for (int l = 0; l < p.grid_num; ++l) {
-        slot += (double)p.maxi[l] * p.maxj[l] * p.maxk[l] * 2 + 2.0 * ((double)p.maxj[l] * p.maxk[l] + (double)p.maxi[l] * p.maxk[l] +
-                                      (double)p.maxi[l] * p.maxj[l]) * 2;
+        // coordinates with their halo, walls
+        slot += (p.maxi[l] + 2.0) * (p.maxj[l] + 2.0) * (p.maxk[l] + 2.0) * 2;
+        slot += 2.0 * ((double)p.maxj[l] * p.maxk[l] + (double)p.maxi[l] * p.maxk[l] + (double)p.maxi[l] * p.maxj[l]) * 2;
     }
     const int nB = p.grey ? p.grey_nB : p.nB, nT = p.grey ? p.grey_nT : p.nT, nQ = p.grey ? 1 : p.nQ;
     const double tabs = (double)nB * nQ * nT * (4 + 4 + sizeof(KIRow<float>)) + (double)nB * nT * 8;
