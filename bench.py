@@ -21,7 +21,7 @@ Legs on one GPU (skipped with --no-legs):
          max|Q| is 1%: solves/s and bundles/s at that tolerance;
   batched  64 uneven problems (grids 16..96 per axis, half grey, half
          narrow-band 20-100 bands, photmax 32/128/512): plain one solve per
-         launch vs one persistent launch from a CUDA graph vs the
+         launch vs all side by side from a CUDA graph vs the
          continuous-batching server, solves/s by wall clock;
   batched_small  the same with edges 16..32 and photmax 32/128;
   dns_source  the DNS coupling kernel (Q, sigma -> Qnew, Varnew, Knew,
@@ -520,7 +520,7 @@ def batch_setup(dev, n=64, edges=(16, 24, 32, 48, 64, 96), photmaxes=(32, 128, 5
 
 def leg_batched(dev, passes=2, tol=None, max_bundles=2.5e11, served=True, warm=True, **mix):
     """Plain (one solve per launch, host arrays in and out, one after the
-    other) vs batched (every solve in one persistent launch replayed from a
+    other) vs batched (a march per solve, side by side, replayed from a
     CUDA graph) vs served (all submitted to the continuous-batching server at
     once) on the uneven mix.  Wall clock per pass of all 64 solves.  With
     `tol`, every problem first runs a pilot at its recipe photmax and then

@@ -95,7 +95,8 @@ typedef struct rc_params {
     double stefan;                      /* param.h:85 */
     float toll, tollS;                  /* param.h:86-87 transmissivity cutoffs */
     int bd[6];                          /* param.h:95-100 */
-    /* grey-gas constants, NarrowBand.h:214-219 */
+    /* grey-gas constants, NarrowBand.h:214-219; with grey_nT > 256 rows a
+     * temperature beyond row 255 is an error of the solve (RC_E_RANGE) */
     int grey_nT, grey_nB;
     float abscoeff, Tmins, wvmax;
     /* narrow-band table dimensions, NarrowBand.h:189-191 */
@@ -147,7 +148,9 @@ int rc_params_default(rc_params *p);
 /* Parse an existing param.h and (optional) NarrowBand.h: #define lines,
  * the maxi/maxj/maxk/maxs initialisers and their #if grid_num branches. */
 int rc_params_from_headers(const char *param_h, const char *narrowband_h, rc_params *p);
-/* Check a parameter set; returns RC_E_INVALID with a message on failure. */
+/* Check a parameter set; returns RC_E_INVALID with a message on failure.
+ * Limits: edges of at most 65535 cells, fewer than 2^31 cells in all levels
+ * (2^32 with the layer of halo cells round each), 2^20 bands, 2^11 g points. */
 int rc_params_validate(const rc_params *p, char *msg, size_t msglen);
 
 /* ---------------- tables ---------------- */

@@ -392,10 +392,9 @@ struct Impl : ImplBase {
     // the second slot's memory is pinned when a second solve is first in
     // flight.  Pinning costs about 1 ms a megabyte, so a program that solves
     // one field at a time, takes floats or collects on the device does not
-    // pay for what it does not use.  (Create and first solve, ms, every slot
-    // with a block from the start / now: 64x64x16
-    // cells 8.5 and 1.8 / 4.5 and 1.4 collected on the device; grey 32^3 6.3
-    // and 0.8 / 5.7 and 0.8; 64^3 11.1 and 6.3 / 8.5 and 6.3.)
+    // pay for what it does not use.  (Create and first solve, ms, medians of
+    // 32, every slot with a block from the start / now: 64x64x16 cells 8.5 + 1.8
+    // / 4.5 + 4.3, grey 32^3 6.4 + 0.8 / 5.7 + 0.8, 64^3 11.1 + 6.3 / 8.5 + 6.3.)
     static constexpr size_t kStageAll = (size_t)2 << 20, kPinRoom = (size_t)2 << 20;
     unsigned char *h_stage = nullptr;
     bool stage_tried = false, stage_own = false;
@@ -979,7 +978,8 @@ struct Impl : ImplBase {
         if (!(c->prio_thr > 0.f) || nt < 1 || nt > kPrioMaxTiles) return RC_OK;
         // with a warp for every tile all start at once: no order to change
         // (first run of a batch of 96 solves of 8^3: 8.5 ms with lists, 7.4
-        // without; 16^3 grey the same either way)
+        // without; 16^3 grey, and batches whose members share the GPU, the same
+        // either way: 64 solves of 16^3 3.7 ms of march, of 12-20 6.8)
         int blocks = 0;
         int rc = resident_blocks(c->block, d.rpt, c->minb, blocks);
         if (rc) return rc;

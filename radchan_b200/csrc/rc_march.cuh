@@ -188,8 +188,10 @@ __device__ __forceinline__ int ring_at(int i) { return i < kRing ? i : i - kRing
 // SCAT: the variant for media with scattering particles.  MINB: the occupancy
 // knob.  Registers of its values: 128 lets two 256-thread blocks onto an SM, 72
 // seven 128-thread blocks, 64 four 256-thread blocks.  72 is the default: 28
-// warps and no more than 24 bytes of spill (64^3, photmax 256: 22.1 ms, with
-// 64 registers 24.2, with 80 and 24 warps 23.3).
+// warps and 24 bytes of spill, 40 with SCAT (64^3, photmax 256: 22.1 ms, with
+// 64 registers 24.2, with 80 and 24 warps 23.3; with scattering coefficients
+// of 0.1-1 1/m 37.2 ms, with 64 registers 40.0, with 128 43.0).  FP64 fits 128
+// (64 and 72 spill 550-750 bytes: 48x40x32 2.5 ms, 3.2 and 3.0).
 constexpr int march_regs(int minb) { return minb >= 4 ? 64 : minb == 3 ? 72 : 128; }
 
 template <typename R, int MINB, bool SCAT>
@@ -306,8 +308,8 @@ __global__ void __launch_bounds__(256) __maxnreg__(march_regs(MINB)) k_march(con
             }
             nbund += valid;
             // with particles, draw 1 (scatter_first_lnu, written out: the
-            // call form spilled) before the emission itself: little is live
-            // then, so the variant fits the register budget without spilling
+            // call form spilled more) before the emission itself: little is
+            // live then, and the variant spills 40 bytes in all
             R lnu = (R)0;
             if constexpr (SCAT) {
                 if (S.nA > 0) {
